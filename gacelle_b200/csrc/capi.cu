@@ -368,6 +368,13 @@ static DevProtocol make_protocol(const gx_model* m, int id, int np, int nm, cons
         P.lb[i] = lb ? (float)lb[i] : 0.0f;
         P.ub[i] = ub ? (float)ub[i] : 1.0f;
     }
+    if (id == kNEXI || id == kNEXI2)
+        for (int i = 0; i < P.nx && P.nx <= kNodeTab; i += 2) {
+            float2 x2, w, wx2, wp2;
+            nexi_node(P.nx, P.h, i, x2, w, wx2, wp2);
+            P.node_a[i / 2] = float4{x2.x, x2.y, w.x, w.y};
+            P.node_b[i / 2] = float4{wx2.x, wx2.y, wp2.x, wp2.y};
+        }
     if (m->kind == GX_MODEL_NEXI_RICE) {
         P.rice = 1;
         for (int i = 1; i < kRiceNodes - 1; ++i) {  // t_i = i pi / 33 (mybesseli nodes)

@@ -23,6 +23,7 @@ constexpr int kMaxFA = 16;
 constexpr int kMaxShell = 64;
 constexpr int kMaxParam = 6;  // fitted parameters + noise
 constexpr int kMaxMeas = 128;
+constexpr int kNodeTab = 128;  // NEXI trapezoid nodes that the protocol tabulates
 
 enum ModelId { kR2S = 1, kR1R2S = 2, kNEXI = 3, kNEXI2 = 4 };
 constexpr int kRiceNodes = 34;  // mybesseli trapezoid nodes (NEXI/gpuNEXIrice.m:752)
@@ -54,6 +55,12 @@ struct DevProtocol {
     int rice;
     float rice_cm1[kRiceNodes - 2];
     float rice_s2[kRiceNodes - 2];
+    // NEXI trapezoid nodes in pairs (2i, 2i + 1), nx <= kNodeTab: x^2 and the
+    // weight w (1, 1/2 at the ends, 0 for the node that pads an odd nx) as
+    // (x2, x2, w, w), and (w x2, w x2, w p2, w p2) with p2 = (3 x^2 - 1) / 2;
+    // rounded as nexi_node rounds them
+    float4 node_a[kNodeTab / 2];
+    float4 node_b[kNodeTab / 2];
 };
 
 // ---------------------------------------------------------------------------
@@ -632,14 +639,55 @@ __device__ __forceinline__ void model_r1r2s(const DevProtocol& P, const float* t
     }
 }
 
+#endif  // __CUDACC__
+
+// Nodes i, i + 1 of the NEXI trapezoid (i even): x^2, the weight w, w x^2 and
+// w (3 x^2 - 1) / 2.  The node index is an exact float (below 2^24).
+GX_HD void nexi_node(int nx, float h, int i, float2& x2, float2& w, float2& wx2, float2& wp2) {
+    const float x0 = (float)i * h, x1 = (float)(i + 1) * h;
+    x2 = float2{x0 * x0, x1 * x1};
+    w = float2{(i == 0 || i == nx - 1) ? 0.5f : 1.0f, i + 1 >= nx ? 0.0f : (i + 1 == nx - 1 ? 0.5f : 1.0f)};
+    wx2 = float2{w.x * x2.x, w.y * x2.y};
+    wp2 = float2{w.x * fmaf(1.5f, x2.x, -0.5f), w.y * fmaf(1.5f, x2.y, -0.5f)};
+}
+
+#if defined(__CUDACC__)
+
 // NEXI narrow-pulse Karger model (NEXI/gpuNEXI.m:902-996, M at :1090-1097):
 // per shell j, S_j = trapz_x M(x) over x = linspace(0,1,nx); lmax = 2 adds
-// Sl2_j = p2 |trapz_x M (3x^2-1)/2|; finally min(S,1).  The tangent sums per
-// node are reduced to the five intermediate partials (f, d1, d2, r1, r2) and
-// chained to (fa, Da, De, ra) once per shell.
-template <bool LMAX2, class Acc, int NP>
-__device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const float* th, const VoxAux& va,
-                                                Acc& acc) {
+// Sl2_j = p2 |trapz_x M (3x^2-1)/2|; finally min(S,1).
+//
+// Per node, with L1 = r1 + r2 + d2 + d1, s = r1 - r2 - d2 + d1 and
+// L2 = sqrt(s^2 + 4 r1 r2) (twice the reference's l1 and l2; the factors of
+// two are exact, so the roundings are those of the halved forms),
+// R = 1 / L2, P = (f d1 + (1-f) d2 - (L1 - L2)/2) R, e+- = exp(-(L1 +- L2)/2):
+//   M = P e+ + (1-P) e-.
+// Adjoint (Mbar = 1), with Nb = (e+ - e-) R, U = (1-P) e- and
+//   W = ((2U - M) + Nb (1 - 2P)) R      (= 4 dM/dQ, Q = L2^2):
+//   dM/df = Nb (d1 - d2),          dM/dd1 = f Nb + (s W - M - Nb)/2,
+//   dM/dd2 = (1-f) Nb - (s W + M + Nb)/2,
+//   dM/dr1 = r2 W + (s W - M - Nb)/2, dM/dr2 = r1 W - (s W + M + Nb)/2.
+// These are linear in Nb, W, M and t = s W - M with coefficients that are
+// constant over a shell's nodes (d1 = b Da x^2), so the loop keeps six sums
+// (M, Nb, W, t, x^2 Nb, x^2 t) and the five partials are formed from them
+// once per shell: 28 pair instructions of FP32 arithmetic per node pair.
+// The nodes go in pairs (i, i+1) on the two lanes of pair instructions, the
+// sums kept per lane and folded at the end; ptxas may fuse a pair multiply
+// into the following pair add, and this is the model's only form, so every
+// path rounds alike.
+//
+// Bound: the FMA pipe (28 pair instructions of 2 cycles a warp and scheduler
+// against 48 cycles of the SFU's 6 operations) with the adjoint, the SFU
+// without it (17 pair instructions).  Measured, per-node partials with the
+// node positions recomputed in the loop (62 pair instructions) -> six sums
+// and tabulated nodes: 328,050 voxels x 24 shells x 14 nodes, MSE, 229 ->
+// 157 us an iteration; 100,003 voxels x 100 nodes, Rician loss, 514 -> 323
+// us (FMA pipe 67 %, SFU 55 % active); Goodman-Weare steps of 20,000 voxels
+// x 64 walkers 435 -> 355 us (SFU 82 %).  Nodes beyond kNodeTab are computed in
+// the loop.  Register caps of 64-96 and an unrolled node loop moved the
+// fits by -4 to +3 % either way and are not used.
+template <bool LMAX2, bool TAB, class Acc, int NP>
+__device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* th, const VoxAux& va, Acc& acc) {
     const float EPS = 1e-8f;
     float fa_in = th[0];
     float f = fmaxf(fa_in, EPS);
@@ -653,6 +701,9 @@ __device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const floa
     int nx = P.nx;
     float h = P.h;
     int nsh = P.n_shell;
+    const float2 z2 = make_float2(0.f, 0.f), one = bcast2(1.0f), two = bcast2(2.0f), mtwo = bcast2(-2.0f);
+    const float2 mhalf = bcast2(-0.5f), mexp = bcast2(-0.5f * kLog2e);  // exp(-L/2) = 2^(-L log2(e)/2)
+    const float2 f2 = bcast2(f);
     for (int j = 0; j < nsh; ++j) {
         float b = P.bval[j], D = P.delta[j];
         float d2 = b * De;
@@ -663,90 +714,75 @@ __device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const floa
         float q4 = 4.0f * r1 * r2;
         float bDa = b * Da;
         float fd2 = omf * d2;
-        // nodes in pairs (i, i+1) on the two lanes of pair instructions, an
-        // odd node count padded with a node of weight 0; per lane the
-        // operations of a node at a time (ptxas may fuse a pair multiply
-        // into the following pair add; this is the model's only form, so
-        // every path rounds alike), the sums kept per lane and folded at
-        // the end
-        const float2 z2 = make_float2(0.f, 0.f), half = bcast2(0.5f), one = bcast2(1.0f), two = bcast2(2.0f);
-        const float2 bDa2 = bcast2(bDa), base2 = bcast2(base), q42 = bcast2(q4), c12 = bcast2(c1);
-        const float2 f2 = bcast2(f), fd22 = bcast2(fd2), d22 = bcast2(d2), omf2 = bcast2(omf);
-        const float2 r2x4 = bcast2(4.0f * r2), r1x4 = bcast2(4.0f * r1);
-        float2 S0p = z2, Sfp = z2, Sd1p = z2, Sd2p = z2, Sr1p = z2, Sr2p = z2;
-        float2 T0p = z2, Tfp = z2, Td1p = z2, Td2p = z2, Tr1p = z2, Tr2p = z2;
-        // node indices (i, i+1) carried as exact floats (integers below 2^24),
-        // so the loop converts no integer to float: conversions share the
-        // SFU's issue rate with the rsqrt and the exponentials of the node
-        float2 fi = make_float2(0.0f, 1.0f);
-        for (int i = 0; i < nx; i += 2, fi = add2(fi, two)) {
-            const float2 x = mul2(fi, bcast2(h));
-            const float2 x2 = mul2(x, x);
+        const float2 bDa2 = bcast2(bDa), base2 = bcast2(base), q42 = bcast2(q4), c12 = bcast2(c1), fd22 = bcast2(fd2);
+        float2 S0p = z2, Ap = z2, Bp = z2, Tp = z2, A2p = z2, Gp = z2;
+        float2 S0q = z2, Aq = z2, Bq = z2, Tq = z2, A2q = z2, Gq = z2;  // weighted with p2 (lmax 2)
+        for (int i = 0; i < nx; i += 2) {
+            float2 x2, wt, wx2, wp2;
+            if constexpr (TAB) {
+                const float4 na = P.node_a[i >> 1], nb = P.node_b[i >> 1];
+                x2 = make_float2(na.x, na.y);
+                wt = make_float2(na.z, na.w);
+                wx2 = make_float2(nb.x, nb.y);
+                wp2 = make_float2(nb.z, nb.w);
+            } else {
+                nexi_node(nx, h, i, x2, wt, wx2, wp2);
+            }
             const float2 d1 = mul2(bDa2, x2);
             const float2 s = add2(base2, d1);
             const float2 Q = fma2(s, s, q42);
             const float2 rs = make_float2(rsqrtf(Q.x), rsqrtf(Q.y));
-            const float2 l2raw = mul2(mul2(half, Q), rs);
-            const bool ax = l2raw.x > EPS, ay = l2raw.y > EPS;
-            const float2 l2 = make_float2(ax ? l2raw.x : EPS, ay ? l2raw.y : EPS);
-            const float2 rs2 = mul2(two, rs);
-            const float2 inv_l2 = make_float2(ax ? rs2.x : 1.0f / EPS, ay ? rs2.y : 1.0f / EPS);
-            const float2 l1 = mul2(half, add2(c12, d1));
-            const float2 lm = sub2(l1, l2), lp = add2(l1, l2);
-            const float2 N = sub2(fma2(f2, d1, fd22), lm);
-            const float2 Pp = mul2(mul2(half, N), inv_l2);
-            const float2 em = make_float2(__expf(-lm.x), __expf(-lm.y));
-            const float2 ep = make_float2(__expf(-lp.x), __expf(-lp.y));
+            // l2 = max(sqrt(Q)/2, eps); a non-number (Q = 0 or infinite) takes eps
+            const float2 L2r = mul2(Q, rs);
+            const float2 L2 = make_float2(fmaxf(L2r.x, 2.0f * EPS), fmaxf(L2r.y, 2.0f * EPS));
+            const float2 R = make_float2(fminf(rs.x, 0.5f / EPS), fminf(rs.y, 0.5f / EPS));
+            const float2 L1 = add2(c12, d1);
+            const float2 LM = sub2(L1, L2), LP = add2(L1, L2);
+            const float2 N = fma2(mhalf, LM, fma2(f2, d1, fd22));
+            const float2 Pp = mul2(N, R);
+            const float2 xm = mul2(LM, mexp), xp = mul2(LP, mexp);
+            const float2 em = make_float2(ex2_ftz(xm.x), ex2_ftz(xm.y));
+            const float2 ep = make_float2(ex2_ftz(xp.x), ex2_ftz(xp.y));
             const float2 omP = sub2(one, Pp);
-            const float2 M = fma2(Pp, ep, mul2(omP, em));
-            // reverse sweep with Mbar = 1
-            const float2 Ppb = sub2(ep, em);
-            const float2 lpb = mul2(make_float2(-Pp.x, -Pp.y), ep);
-            float2 lmb = mul2(make_float2(-omP.x, -omP.y), em);
-            const float2 Nb = mul2(mul2(half, Ppb), inv_l2);
-            float2 l2b = mul2(mul2(make_float2(-Ppb.x, -Ppb.y), Pp), inv_l2);
-            lmb = sub2(lmb, Nb);
-            const float2 l1b = add2(lpb, lmb);
-            l2b = add2(l2b, sub2(lpb, lmb));
-            const float2 Qbr = mul2(mul2(bcast2(0.125f), l2b), inv_l2);
-            const float2 Qb = make_float2(ax ? Qbr.x : 0.0f, ay ? Qbr.y : 0.0f);
-            const float2 sb = mul2(mul2(two, s), Qb);
-            const float2 hl1 = mul2(half, l1b);
-            const float2 fb = mul2(Nb, sub2(d1, d22));
-            const float2 d1b = add2(add2(mul2(Nb, f2), sb), hl1);
-            const float2 d2b = add2(sub2(mul2(Nb, omf2), sb), hl1);
-            const float2 r1b = add2(add2(mul2(r2x4, Qb), sb), hl1);
-            const float2 r2b = add2(sub2(mul2(r1x4, Qb), sb), hl1);
-            const float2 wt = make_float2((i == 0 || i == nx - 1) ? 0.5f : 1.0f,
-                                          i + 1 >= nx ? 0.0f : (i + 1 == nx - 1 ? 0.5f : 1.0f));
+            const float2 U = mul2(omP, em);
+            const float2 M = fma2(Pp, ep, U);
+            const float2 Nb = mul2(sub2(ep, em), R);
+            const float2 Wr = mul2(fma2(Nb, fma2(mtwo, Pp, one), fma2(two, U, make_float2(-M.x, -M.y))), R);
+            const float2 W = make_float2(rs.x < 0.5f / EPS ? Wr.x : 0.0f, rs.y < 0.5f / EPS ? Wr.y : 0.0f);
+            const float2 t = fma2(s, W, make_float2(-M.x, -M.y));
             S0p = fma2(wt, M, S0p);
-            Sfp = fma2(wt, fb, Sfp);
-            Sd1p = fma2(mul2(wt, x2), d1b, Sd1p);
-            Sd2p = fma2(wt, d2b, Sd2p);
-            Sr1p = fma2(wt, r1b, Sr1p);
-            Sr2p = fma2(wt, r2b, Sr2p);
+            Ap = fma2(wt, Nb, Ap);
+            Bp = fma2(wt, W, Bp);
+            Tp = fma2(wt, t, Tp);
+            A2p = fma2(wx2, Nb, A2p);
+            Gp = fma2(wx2, t, Gp);
             if (LMAX2) {
-                const float2 p2w = mul2(wt, fma2(bcast2(1.5f), x2, bcast2(-0.5f)));
-                T0p = fma2(p2w, M, T0p);
-                Tfp = fma2(p2w, fb, Tfp);
-                Td1p = fma2(mul2(p2w, x2), d1b, Td1p);
-                Td2p = fma2(p2w, d2b, Td2p);
-                Tr1p = fma2(p2w, r1b, Tr1p);
-                Tr2p = fma2(p2w, r2b, Tr2p);
+                const float2 wp2x2 = mul2(wp2, x2);
+                S0q = fma2(wp2, M, S0q);
+                Aq = fma2(wp2, Nb, Aq);
+                Bq = fma2(wp2, W, Bq);
+                Tq = fma2(wp2, t, Tq);
+                A2q = fma2(wp2x2, Nb, A2q);
+                Gq = fma2(wp2x2, t, Gq);
             }
         }
-        const float S0 = S0p.x + S0p.y, Sf = Sfp.x + Sfp.y, Sd1 = Sd1p.x + Sd1p.y, Sd2 = Sd2p.x + Sd2p.y;
-        const float Sr1 = Sr1p.x + Sr1p.y, Sr2 = Sr2p.x + Sr2p.y;
-        const float T0 = T0p.x + T0p.y, Tf = Tfp.x + Tfp.y, Td1 = Td1p.x + Td1p.y, Td2 = Td2p.x + Td2p.y;
-        const float Tr1 = Tr1p.x + Tr1p.y, Tr2 = Tr2p.x + Tr2p.y;
-        float r2_f = rice ? (omf > EPS ? r1 / (omf * omf) : r1 / EPS) : r1 / (omf * omf);
+        const float r2_f = rice ? (omf > EPS ? r1 / (omf * omf) : r1 / EPS) : r1 / (omf * omf);
+        // d(sum)/d(fa, Da, De, ra) times h from the six sums
+        auto partials = [&](float S0, float A, float B, float T, float A2, float G, float (&g)[4]) {
+            const float up = 0.5f * (T - A), um = -(0.5f * (T + A) + S0);
+            const float Sr2 = fmaf(r1, B, um);
+            g[0] = gate * h * (fmaf(bDa, A2, -d2 * A) + Sr2 * r2_f);
+            g[1] = h * fmaf(f - 0.5f, A2, 0.5f * G) * b;
+            g[2] = h * fmaf(omf, A, um) * b;
+            g[3] = h * (fmaf(r2, B, up) + Sr2 * rf) * D;
+        };
         {
+            const float S0 = S0p.x + S0p.y;
             float S = S0 * h;
-            float dS[NP];
-            dS[0] = gate * h * (Sf + Sr2 * r2_f);
-            dS[1] = h * Sd1 * b;
-            dS[2] = h * Sd2 * b;
-            dS[3] = h * (Sr1 + Sr2 * rf) * D;
+            float g[4], dS[NP];
+            partials(S0, Ap.x + Ap.y, Bp.x + Bp.y, Tp.x + Tp.y, A2p.x + A2p.y, Gp.x + Gp.y, g);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dS[k] = g[k];
             if (NP > 4) dS[NP - 1] = 0.0f;
             if (rice) {  // Rician floor correction (NEXI/gpuNEXIrice.m:653)
                 float dM1;
@@ -762,15 +798,15 @@ __device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const floa
             acc.add(j, S, dS);
         }
         if (LMAX2) {
-            float p2 = th[NP - 1];
-            float T = T0 * h;
-            float sg = (float)((T > 0.0f) - (T < 0.0f));
+            const float p2 = th[NP - 1];
+            const float T0 = S0q.x + S0q.y;
+            const float T = T0 * h;
+            const float sg = p2 * (float)((T > 0.0f) - (T < 0.0f));
             float S = p2 * fabsf(T);
-            float dS[NP];
-            dS[0] = gate * p2 * sg * h * (Tf + Tr2 * r2_f);
-            dS[1] = p2 * sg * h * Td1 * b;
-            dS[2] = p2 * sg * h * Td2 * b;
-            dS[3] = p2 * sg * h * (Tr1 + Tr2 * rf) * D;
+            float g[4], dS[NP];
+            partials(T0, Aq.x + Aq.y, Bq.x + Bq.y, Tq.x + Tq.y, A2q.x + A2q.y, Gq.x + Gq.y, g);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dS[k] = sg * g[k];
             dS[NP - 1] = fabsf(T);
             if (S > 1.0f) {
                 S = 1.0f;
@@ -780,6 +816,12 @@ __device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const floa
             acc.add(nsh + j, S, dS);
         }
     }
+}
+
+template <bool LMAX2, class Acc, int NP>
+__device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const float* th, const VoxAux& va, Acc& acc) {
+    if (P.nx <= kNodeTab) nexi_shells<LMAX2, true, Acc, NP>(P, th, va, acc);
+    else nexi_shells<LMAX2, false, Acc, NP>(P, th, va, acc);
 }
 
 // UNROLL: unrolled protocol loops where a caller's register budget allows

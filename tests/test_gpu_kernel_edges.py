@@ -1,0 +1,53 @@
+"""Edges of the kernels' tiles and dispatch rules, each against the FP64 oracle
+or a plain restatement: remainders, the smallest and the largest of a range,
+and both sides of each rule."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from gacelle_b200 import _lib
+from gacelle_b200 import askadam_solver as gx_askadam
+
+from helpers import NAMES, bounds, fitting, models, random_theta
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["nexi", "nexi2"])
+@pytest.mark.parametrize("nx", [2, 3, 127, 128, 129])
+def test_nexi_node_table_and_loop(ctx, kind, nx):
+    """Signal and gradient around the largest tabulated node count, with odd
+    and even counts.  Bars: of the forward and gradient parity tests, the
+    signal's relative to the sum of the magnitudes of its trapezoid's terms:
+    that is the signal itself for l = 0, and at most p2 times the l = 0 signal
+    for the signed l = 2 integral (its weights are at most 1)."""
+    rng = np.random.default_rng(nx)
+    n = 65
+    gxm, om = models(kind, nx=nx)
+    lb, ub = bounds(kind)
+    th = random_theta(kind, n, rng).astype(np.float32)
+    s = oracle.forward(om, th.astype(np.float64))
+    out = np.zeros(s.shape, np.float32)
+    _lib.check(_lib.lib().gx_forward(ctx.ptr, C.byref(gxm.s), _lib.MEM_HOST, th.ctypes.data, None, n,
+                                     out.ctypes.data))
+    scale = np.abs(s)
+    if kind == "nexi2":
+        scale[24:] = np.maximum(scale[24:], th[4] * scale[:24])
+    assert np.max(np.abs(out - s) / np.maximum(scale, 1e-3)) < 2e-5
+    y = (s + 0.02 * rng.standard_normal(s.shape)).astype(np.float32)
+    f = fitting(lossFunction="mse")
+    opts = gx_askadam.build_opts(f, NAMES[kind], lb, ub)
+    vol = _lib.GxVolume()
+    vol.dims[0], vol.dims[1], vol.dims[2] = n, 1, 1
+    vol.nvox = n
+    vol.data = y.ctypes.data_as(_lib._fp)
+    g, loss = np.zeros_like(th), C.c_double()
+    _lib.check(_lib.lib().gx_model_gradient(ctx.ptr, C.byref(gxm.s), _lib.MEM_HOST, C.byref(vol), C.byref(opts),
+                                            th.ctypes.data, g.ctypes.data, None, C.byref(loss), None, None))
+    Lo, go, _, _, _ = oracle.model_gradient(om, oracle.Volume(y.astype(np.float64)), oracle.adam_opts(lb, ub, f),
+                                            th.astype(np.float64))
+    assert abs(loss.value - Lo) <= 1e-5 * abs(Lo) + 1e-7
+    for k in range(th.shape[0]):
+        assert np.max(np.abs(g[k] - go[k])) <= 1e-3 * np.max(np.abs(go[k])) + 1e-12
