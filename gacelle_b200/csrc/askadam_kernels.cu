@@ -20,6 +20,7 @@
 // initialise_parameter :368-412, update_parameters :673-691,
 // unscale_parameters :1063-1075), utils/spatial_total_variation.m.
 #include <climits>
+#include <type_traits>
 
 #include "gx_internal.h"
 
@@ -158,6 +159,12 @@ __device__ __forceinline__ void fused_body(const AdamParams& a, int e_begin, int
         for (int f = 0; f < a.P.n_fa; ++f) sincosf(b1 * a.P.fa_rad[f], &s_sa[f * B + tid], &s_ca[f * B + tid]);
     VoxAux va{b1, s_sa + tid, s_ca + tid, B};
     va.sigma = voxel_sigma(a, v);
+    if constexpr (kIsNexi<MODEL>)
+        if (a.node_smem) {
+            NexiNodes* s_nodes = reinterpret_cast<NexiNodes*>(s_ca + a.P.n_fa * B);
+            stage_nodes(a.nodes, s_nodes);
+            va.nodes = s_nodes;
+        }
     LossAux aux = make_loss_aux(voxel_sigma(a, v));
     __syncthreads();
 
@@ -271,9 +278,19 @@ __global__ void __maxnreg__(80) fused_kernel_r1r2s(AdamParams a, int e_begin, in
     fused_body<kR1R2S, LOSS, STATS>(a, e_begin, e_end, update_last, record);
 }
 
+// NEXI with lmax 0: registers capped at 96 (20 warps an SM; uncapped up to
+// 128, 16 warps): 328,050 voxels x 14 nodes, MSE, 195 -> 187 us an iteration,
+// 100,003 voxels x 100 nodes, Rician loss, 429 -> 414 us; 88 and 80 are slower
+// again.  lmax 2 keeps twice the sums and would spill.
+template <int MODEL, int LOSS, bool STATS>
+__global__ void __maxnreg__(96) fused_kernel_nexi(AdamParams a, int e_begin, int e_end, int update_last, int record) {
+    fused_body<MODEL, LOSS, STATS>(a, e_begin, e_end, update_last, record);
+}
+
 template <int MODEL, int LOSS, bool STATS>
 constexpr auto fused_kernel_fn() {
-    if constexpr (MODEL == kR1R2S) return &fused_kernel_r1r2s<LOSS, STATS>;
+    if constexpr (MODEL == kNEXI) return &fused_kernel_nexi<MODEL, LOSS, STATS>;
+    else if constexpr (MODEL == kR1R2S) return &fused_kernel_r1r2s<LOSS, STATS>;
     else return &fused_kernel<MODEL, LOSS, STATS>;
 }
 
@@ -292,6 +309,8 @@ __global__ void tv_step_kernel(AdamParams a, int e, int update, int record, int 
     __shared__ double s_red[2 * 32 * NQ];
     __shared__ DevProtocol s_P;
     stage_protocol(a.P, &s_P);
+    __shared__ __align__(16) unsigned char s_nodes[kIsNexi<MODEL> ? sizeof(NexiNodes) : 16];
+    if constexpr (kIsNexi<MODEL>) stage_nodes(a.nodes, reinterpret_cast<NexiNodes*>(s_nodes));
     __syncthreads();
     const int B = blockDim.x, tid = threadIdx.x;
     const int v = blockIdx.x * B + tid;
@@ -312,6 +331,7 @@ __global__ void tv_step_kernel(AdamParams a, int e, int update, int record, int 
     if (MODEL == kR1R2S)
         for (int f = 0; f < a.P.n_fa; ++f) sincosf(b1 * a.P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
+    if constexpr (kIsNexi<MODEL>) va.nodes = reinterpret_cast<const NexiNodes*>(s_nodes);
     va.sigma = voxel_sigma(a, v);
     float th[NP], dth[NP];
 #pragma unroll
@@ -554,6 +574,7 @@ __global__ void plain_forward_kernel(AdamParams a, PlainBufs b) {
         for (int f = 0; f < a.P.n_fa; ++f) sincosf(b1 * a.P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
     va.sigma = voxel_sigma(a, v);
+    va.nodes = &a.nodes;
     SignalSink<NP> sink{b.signal + v, a.nvtot};
     model_eval<MODEL>(a.P, th, va, sink);
 }
@@ -734,6 +755,7 @@ __global__ void plain_adjoint_kernel(AdamParams a, PlainBufs b) {
         for (int f = 0; f < a.P.n_fa; ++f) sincosf(b1 * a.P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
     va.sigma = voxel_sigma(a, v);
+    va.nodes = &a.nodes;
     DsigAcc<NP> acc;
     acc.ds = b.dsig + v;
     acc.s = a.nvtot;
@@ -865,8 +887,12 @@ __global__ void plain_update_kernel(AdamParams a, PlainBufs b, int e) {
     }
 }
 
+// The node table as a parameter, for the models that have one.
+struct NoNodes {};
+template <int MODEL> using NodesArg = std::conditional_t<kIsNexi<MODEL>, NexiNodes, NoNodes>;
+
 template <int MODEL>
-__global__ void forward_only_kernel(DevProtocol P, const float* theta, const float* b1_, int nvox,
+__global__ void forward_only_kernel(DevProtocol P, NodesArg<MODEL> nodes, const float* theta, const float* b1_, int nvox,
                                     float* signal) {
     constexpr int NP = ModelNP<MODEL>::value;
     int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -878,6 +904,7 @@ __global__ void forward_only_kernel(DevProtocol P, const float* theta, const flo
     if (MODEL == kR1R2S)
         for (int f = 0; f < P.n_fa; ++f) sincosf(b1 * P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
+    if constexpr (kIsNexi<MODEL>) va.nodes = &nodes;
     va.sigma = b1;  // the aux map: b1 (R1R2*) or sigma (NEXI Rician mean)
     SignalSink<NP> sink{signal + v, nvox};
     model_eval<MODEL>(P, th, va, sink);
@@ -894,14 +921,25 @@ __global__ void forward_only_kernel(DevProtocol P, const float* theta, const flo
     default: F<kNEXI2, __VA_ARGS__>; break;                 \
     }
 
+// Adds the node table to a kernel's dynamic shared memory (16-byte aligned
+// behind it) when that fits beside the staged protocol; otherwise the nodes
+// are computed in the loop.
+int nodes_fit(size_t* smem) {
+    const size_t with = (*smem + 15) / 16 * 16 + sizeof(NexiNodes);
+    if (with + sizeof(DevProtocol) + 1024 > kMaxSmemPerBlock) return 0;
+    *smem = with;
+    return 1;
+}
+
 template <int MODEL, int LOSS, bool STATS>
-static cudaError_t fused_dispatch3(const AdamParams& a, int e_begin, int e_end, int update_last,
+static cudaError_t fused_dispatch3(AdamParams a, int e_begin, int e_end, int update_last,
                                    bool record, int block, int nblocks, cudaStream_t s) {
     constexpr int NQ = STATS ? kHistW : 1;
     size_t smem = sizeof(double) * 2 * 32 * NQ +
                   sizeof(float) * (size_t)block * (a.nm * (a.weights ? 2 : 1) + 2 * a.P.n_fa);
     auto k = fused_kernel_fn<MODEL, LOSS, STATS>();
-    if (smem > 48 * 1024) {
+    if (kIsNexi<MODEL>) a.node_smem = nodes_fit(&smem);
+    if (smem + sizeof(DevProtocol) > 48 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;
     }
@@ -1134,11 +1172,13 @@ cudaError_t launch_forward_only(const DevProtocol& P, int model, const float* th
     const int block = 128;
     int nb = (nvox + block - 1) / block;
     if (nb == 0) return cudaSuccess;
+    NexiNodes nodes;
+    make_nodes(P, &nodes);
     switch (model) {
-    case kR2S: forward_only_kernel<kR2S><<<nb, block, 0, s>>>(P, theta, b1, nvox, signal); break;
-    case kR1R2S: forward_only_kernel<kR1R2S><<<nb, block, 0, s>>>(P, theta, b1, nvox, signal); break;
-    case kNEXI: forward_only_kernel<kNEXI><<<nb, block, 0, s>>>(P, theta, b1, nvox, signal); break;
-    default: forward_only_kernel<kNEXI2><<<nb, block, 0, s>>>(P, theta, b1, nvox, signal); break;
+    case kR2S: forward_only_kernel<kR2S><<<nb, block, 0, s>>>(P, NoNodes{}, theta, b1, nvox, signal); break;
+    case kR1R2S: forward_only_kernel<kR1R2S><<<nb, block, 0, s>>>(P, NoNodes{}, theta, b1, nvox, signal); break;
+    case kNEXI: forward_only_kernel<kNEXI><<<nb, block, 0, s>>>(P, nodes, theta, b1, nvox, signal); break;
+    default: forward_only_kernel<kNEXI2><<<nb, block, 0, s>>>(P, nodes, theta, b1, nvox, signal); break;
     }
     ++g_kernel_launches;
     return cudaGetLastError();

@@ -368,13 +368,6 @@ static DevProtocol make_protocol(const gx_model* m, int id, int np, int nm, cons
         P.lb[i] = lb ? (float)lb[i] : 0.0f;
         P.ub[i] = ub ? (float)ub[i] : 1.0f;
     }
-    if (id == kNEXI || id == kNEXI2)
-        for (int i = 0; i < P.nx && P.nx <= kNodeTab; i += 2) {
-            float2 x2, w, wx2, wp2;
-            nexi_node(P.nx, P.h, i, x2, w, wx2, wp2);
-            P.node_a[i / 2] = float4{x2.x, x2.y, w.x, w.y};
-            P.node_b[i / 2] = float4{wx2.x, wx2.y, wp2.x, wp2.y};
-        }
     if (m->kind == GX_MODEL_NEXI_RICE) {
         P.rice = 1;
         for (int i = 1; i < kRiceNodes - 1; ++i) {  // t_i = i pi / 33 (mybesseli nodes)
@@ -385,6 +378,19 @@ static DevProtocol make_protocol(const gx_model* m, int id, int np, int nm, cons
     }
     return P;
 }
+
+namespace gx {
+void make_nodes(const DevProtocol& P, NexiNodes* t) {
+    memset(t, 0, sizeof(*t));
+    if (P.model != kNEXI && P.model != kNEXI2) return;
+    for (int i = 0; i < P.nx && P.nx <= kNodeTab; i += 2) {
+        float2 x2, w, wx2, wp2;
+        nexi_node(P.nx, P.h, i, x2, w, wx2, wp2);
+        t->a[i / 2] = float4{x2.x, x2.y, w.x, w.y};
+        t->b[i / 2] = float4{wx2.x, wx2.y, wp2.x, wp2.y};
+    }
+}
+}  // namespace gx
 
 // ---------------------------------------------------------------------------
 // Host restatement of the reference's per-epoch bookkeeping
@@ -690,6 +696,7 @@ static gx_status adam_setup(AdamJob& J) {
     AdamParams& a = J.a;
     memset(&a, 0, sizeof(a));
     a.P = make_protocol(J.model, J.id, J.np, J.nm, o->lb, o->ub, J.np);
+    make_nodes(a.P, &a.nodes);
     a.nm = J.nm;
     a.np = J.np;
     a.nvtot = J.nvtot;
@@ -1736,6 +1743,7 @@ extern "C" gx_status gx_mcmc(gx_context* c, const gx_model* model, int32_t mem, 
         McmcParams p;
         memset(&p, 0, sizeof(p));
         p.P = make_protocol(model, id, np, nm, nullptr, nullptr, 0);
+        make_nodes(p.P, &p.nodes);
         p.nm = nm; p.nvar = nvar; p.nvox = nv;
         for (int q = 0; q < nvar; ++q) {
             p.lb[q] = (float)o->lb[q];

@@ -55,12 +55,16 @@ struct DevProtocol {
     int rice;
     float rice_cm1[kRiceNodes - 2];
     float rice_s2[kRiceNodes - 2];
-    // NEXI trapezoid nodes in pairs (2i, 2i + 1), nx <= kNodeTab: x^2 and the
-    // weight w (1, 1/2 at the ends, 0 for the node that pads an odd nx) as
-    // (x2, x2, w, w), and (w x2, w x2, w p2, w p2) with p2 = (3 x^2 - 1) / 2;
-    // rounded as nexi_node rounds them
-    float4 node_a[kNodeTab / 2];
-    float4 node_b[kNodeTab / 2];
+};
+
+// NEXI trapezoid nodes in pairs (2i, 2i + 1), nx <= kNodeTab: x^2 and the
+// weight w (1, 1/2 at the ends, 0 for the node that pads an odd nx) as
+// (x2, x2, w, w), and (w x2, w x2, w p2, w p2) with p2 = (3 x^2 - 1) / 2;
+// rounded as nexi_node rounds them.  A kernel parameter, copied to shared
+// memory by the kernels that read it often.
+struct NexiNodes {
+    float4 a[kNodeTab / 2];
+    float4 b[kNodeTab / 2];
 };
 
 // ---------------------------------------------------------------------------
@@ -420,6 +424,7 @@ struct VoxAux {
     const float* ca;          // R1R2*: cos(b1*FA_f)
     int fs;
     float sigma = 1.0f;       // NEXI Rician mean: noise sigma (normalised by b0)
+    const NexiNodes* nodes = nullptr;  // NEXI: the tabulated nodes (nullptr: computed in the loop)
 };
 
 // Rician mean of a noise-free signal S (myriceM1 / myL12 / mybesseli,
@@ -662,30 +667,30 @@ GX_HD void nexi_node(int nx, float h, int i, float2& x2, float2& w, float2& wx2,
 // two are exact, so the roundings are those of the halved forms),
 // R = 1 / L2, P = (f d1 + (1-f) d2 - (L1 - L2)/2) R, e+- = exp(-(L1 +- L2)/2):
 //   M = P e+ + (1-P) e-.
-// Adjoint (Mbar = 1), with Nb = (e+ - e-) R, U = (1-P) e- and
+// Adjoint (Mbar = 1), with Nb = (e+ - e-) R, U = (1-P) e-, a = M + Nb and
 //   W = ((2U - M) + Nb (1 - 2P)) R      (= 4 dM/dQ, Q = L2^2):
-//   dM/df = Nb (d1 - d2),          dM/dd1 = f Nb + (s W - M - Nb)/2,
-//   dM/dd2 = (1-f) Nb - (s W + M + Nb)/2,
-//   dM/dr1 = r2 W + (s W - M - Nb)/2, dM/dr2 = r1 W - (s W + M + Nb)/2.
-// These are linear in Nb, W, M and t = s W - M with coefficients that are
-// constant over a shell's nodes (d1 = b Da x^2), so the loop keeps six sums
-// (M, Nb, W, t, x^2 Nb, x^2 t) and the five partials are formed from them
-// once per shell: 28 pair instructions of FP32 arithmetic per node pair.
+//   2 dM/df  = 2 Nb (d1 - d2),
+//   2 dM/dd1 = 2 f Nb + (s W - a),   2 dM/dd2 = 2 (1-f) Nb - (s W + a),
+//   2 dM/dr1 = 2 r2 W + (s W - a),   2 dM/dr2 = 2 r1 W - (s W + a):
+// 36 FP32 pair instructions per node pair.  (The sums are taken of these
+// per-node values: W, Nb and M summed apart and combined per shell would take
+// 28, but their combinations cancel, and the sums' rounding made d/dra and
+// d/dDe 4-10 times less exact; dM/dd2 and dM/dr1 as differences of the other
+// two, or from (r1 + r2 -+ (d2 - d1)) W - a, had errors up to 1.3 times these.)
 // The nodes go in pairs (i, i+1) on the two lanes of pair instructions, the
 // sums kept per lane and folded at the end; ptxas may fuse a pair multiply
 // into the following pair add, and this is the model's only form, so every
 // path rounds alike.
 //
-// Bound: the FMA pipe (28 pair instructions of 2 cycles a warp and scheduler
+// Bound: the FMA pipe (36 pair instructions of 2 cycles a warp and scheduler
 // against 48 cycles of the SFU's 6 operations) with the adjoint, the SFU
-// without it (17 pair instructions).  Measured, per-node partials with the
-// node positions recomputed in the loop (62 pair instructions) -> six sums
-// and tabulated nodes: 328,050 voxels x 24 shells x 14 nodes, MSE, 229 ->
-// 157 us an iteration; 100,003 voxels x 100 nodes, Rician loss, 514 -> 323
-// us (FMA pipe 67 %, SFU 55 % active); Goodman-Weare steps of 20,000 voxels
-// x 64 walkers 435 -> 355 us (SFU 82 %).  Nodes beyond kNodeTab are computed in
-// the loop.  Register caps of 64-96 and an unrolled node loop moved the
-// fits by -4 to +3 % either way and are not used.
+// without it (17 pair instructions).  Measured, 62 pair instructions with the
+// node positions recomputed in the loop -> this form: 328,050 voxels x 24
+// shells x 14 nodes, MSE, 229 -> 187 us an iteration; 100,003 voxels x 100
+// nodes, Rician loss, 514 -> 414 us; Goodman-Weare steps of 20,000 voxels x 64
+// walkers 435 -> 344 us (SFU 82 % active).  The table is read from shared
+// memory: through the constant bank the same kernels take 2-20 % longer.
+// Nodes beyond kNodeTab are computed in the loop.
 template <bool LMAX2, bool TAB, class Acc, int NP>
 __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* th, const VoxAux& va, Acc& acc) {
     const float EPS = 1e-8f;
@@ -703,7 +708,7 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
     int nsh = P.n_shell;
     const float2 z2 = make_float2(0.f, 0.f), one = bcast2(1.0f), two = bcast2(2.0f), mtwo = bcast2(-2.0f);
     const float2 mhalf = bcast2(-0.5f), mexp = bcast2(-0.5f * kLog2e);  // exp(-L/2) = 2^(-L log2(e)/2)
-    const float2 f2 = bcast2(f);
+    const float2 f2 = bcast2(f), f2x2 = bcast2(2.0f * f), omf2x2 = bcast2(2.0f * omf);
     for (int j = 0; j < nsh; ++j) {
         float b = P.bval[j], D = P.delta[j];
         float d2 = b * De;
@@ -715,12 +720,13 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
         float bDa = b * Da;
         float fd2 = omf * d2;
         const float2 bDa2 = bcast2(bDa), base2 = bcast2(base), q42 = bcast2(q4), c12 = bcast2(c1), fd22 = bcast2(fd2);
-        float2 S0p = z2, Ap = z2, Bp = z2, Tp = z2, A2p = z2, Gp = z2;
-        float2 S0q = z2, Aq = z2, Bq = z2, Tq = z2, A2q = z2, Gq = z2;  // weighted with p2 (lmax 2)
+        const float2 bDax2 = bcast2(2.0f * bDa), md2x2 = bcast2(-2.0f * d2), r1x2 = bcast2(2.0f * r1), r2x2 = bcast2(2.0f * r2);
+        float2 S0p = z2, Sfp = z2, Sd1p = z2, Sd2p = z2, Sr1p = z2, Sr2p = z2;
+        float2 S0q = z2, Sfq = z2, Sd1q = z2, Sd2q = z2, Sr1q = z2, Sr2q = z2;  // weighted with p2 (lmax 2)
         for (int i = 0; i < nx; i += 2) {
             float2 x2, wt, wx2, wp2;
             if constexpr (TAB) {
-                const float4 na = P.node_a[i >> 1], nb = P.node_b[i >> 1];
+                const float4 na = va.nodes->a[i >> 1], nb = va.nodes->b[i >> 1];
                 x2 = make_float2(na.x, na.y);
                 wt = make_float2(na.z, na.w);
                 wx2 = make_float2(nb.x, nb.y);
@@ -749,38 +755,42 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
             const float2 Nb = mul2(sub2(ep, em), R);
             const float2 Wr = mul2(fma2(Nb, fma2(mtwo, Pp, one), fma2(two, U, make_float2(-M.x, -M.y))), R);
             const float2 W = make_float2(rs.x < 0.5f / EPS ? Wr.x : 0.0f, rs.y < 0.5f / EPS ? Wr.y : 0.0f);
-            const float2 t = fma2(s, W, make_float2(-M.x, -M.y));
+            const float2 av = add2(M, Nb), ma = make_float2(-av.x, -av.y);
+            const float2 dd = fma2(bDax2, x2, md2x2);            // 2 (d1 - d2)
+            const float2 fb = mul2(Nb, dd);                      // each derivative times two
+            const float2 gp = fma2(s, W, ma), gm = fma2(make_float2(-s.x, -s.y), W, ma);
+            const float2 d1b = fma2(f2x2, Nb, gp), d2b = fma2(omf2x2, Nb, gm);
+            const float2 r1b = fma2(r2x2, W, gp), r2b = fma2(r1x2, W, gm);
             S0p = fma2(wt, M, S0p);
-            Ap = fma2(wt, Nb, Ap);
-            Bp = fma2(wt, W, Bp);
-            Tp = fma2(wt, t, Tp);
-            A2p = fma2(wx2, Nb, A2p);
-            Gp = fma2(wx2, t, Gp);
+            Sfp = fma2(wt, fb, Sfp);
+            Sd1p = fma2(wx2, d1b, Sd1p);
+            Sd2p = fma2(wt, d2b, Sd2p);
+            Sr1p = fma2(wt, r1b, Sr1p);
+            Sr2p = fma2(wt, r2b, Sr2p);
             if (LMAX2) {
-                const float2 wp2x2 = mul2(wp2, x2);
                 S0q = fma2(wp2, M, S0q);
-                Aq = fma2(wp2, Nb, Aq);
-                Bq = fma2(wp2, W, Bq);
-                Tq = fma2(wp2, t, Tq);
-                A2q = fma2(wp2x2, Nb, A2q);
-                Gq = fma2(wp2x2, t, Gq);
+                Sfq = fma2(wp2, fb, Sfq);
+                Sd1q = fma2(mul2(wp2, x2), d1b, Sd1q);
+                Sd2q = fma2(wp2, d2b, Sd2q);
+                Sr1q = fma2(wp2, r1b, Sr1q);
+                Sr2q = fma2(wp2, r2b, Sr2q);
             }
         }
         const float r2_f = rice ? (omf > EPS ? r1 / (omf * omf) : r1 / EPS) : r1 / (omf * omf);
-        // d(sum)/d(fa, Da, De, ra) times h from the six sums
-        auto partials = [&](float S0, float A, float B, float T, float A2, float G, float (&g)[4]) {
-            const float up = 0.5f * (T - A), um = -(0.5f * (T + A) + S0);
-            const float Sr2 = fmaf(r1, B, um);
-            g[0] = gate * h * (fmaf(bDa, A2, -d2 * A) + Sr2 * r2_f);
-            g[1] = h * fmaf(f - 0.5f, A2, 0.5f * G) * b;
-            g[2] = h * fmaf(omf, A, um) * b;
-            g[3] = h * (fmaf(r2, B, up) + Sr2 * rf) * D;
+        // derivatives of the shell's signal with respect to (fa, Da, De, ra)
+        const float hh = 0.5f * h;
+        auto partials = [&](float2 Sf, float2 Sd1, float2 Sd2, float2 Sr1, float2 Sr2, float (&g)[4]) {
+            const float r2s = Sr2.x + Sr2.y;
+            g[0] = gate * hh * ((Sf.x + Sf.y) + r2s * r2_f);
+            g[1] = hh * (Sd1.x + Sd1.y) * b;
+            g[2] = hh * (Sd2.x + Sd2.y) * b;
+            g[3] = hh * ((Sr1.x + Sr1.y) + r2s * rf) * D;
         };
         {
             const float S0 = S0p.x + S0p.y;
             float S = S0 * h;
             float g[4], dS[NP];
-            partials(S0, Ap.x + Ap.y, Bp.x + Bp.y, Tp.x + Tp.y, A2p.x + A2p.y, Gp.x + Gp.y, g);
+            partials(Sfp, Sd1p, Sd2p, Sr1p, Sr2p, g);
 #pragma unroll
             for (int k = 0; k < 4; ++k) dS[k] = g[k];
             if (NP > 4) dS[NP - 1] = 0.0f;
@@ -804,7 +814,7 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
             const float sg = p2 * (float)((T > 0.0f) - (T < 0.0f));
             float S = p2 * fabsf(T);
             float g[4], dS[NP];
-            partials(T0, Aq.x + Aq.y, Bq.x + Bq.y, Tq.x + Tq.y, A2q.x + A2q.y, Gq.x + Gq.y, g);
+            partials(Sfq, Sd1q, Sd2q, Sr1q, Sr2q, g);
 #pragma unroll
             for (int k = 0; k < 4; ++k) dS[k] = sg * g[k];
             dS[NP - 1] = fabsf(T);
@@ -820,7 +830,7 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
 
 template <bool LMAX2, class Acc, int NP>
 __device__ __forceinline__ void model_nexi_impl(const DevProtocol& P, const float* th, const VoxAux& va, Acc& acc) {
-    if (P.nx <= kNodeTab) nexi_shells<LMAX2, true, Acc, NP>(P, th, va, acc);
+    if (va.nodes && P.nx <= kNodeTab) nexi_shells<LMAX2, true, Acc, NP>(P, th, va, acc);
     else nexi_shells<LMAX2, false, Acc, NP>(P, th, va, acc);
 }
 
@@ -865,6 +875,14 @@ __device__ __forceinline__ void stage_protocol(const DevProtocol& P, DevProtocol
     int* dst = reinterpret_cast<int*>(s_P);
     for (int i = threadIdx.x; i < (int)(sizeof(DevProtocol) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
 }
+
+__device__ __forceinline__ void stage_nodes(const NexiNodes& src, NexiNodes* dst) {
+    const float4* f = src.a;
+    float4* t = dst->a;
+    for (int i = threadIdx.x; i < (int)(sizeof(NexiNodes) / sizeof(float4)); i += blockDim.x) t[i] = f[i];
+}
+
+template <int MODEL> constexpr bool kIsNexi = MODEL == kNEXI || MODEL == kNEXI2;
 
 // unscale_parameters (utils/askadam.m:1063-1075) and its derivative: the
 // logistic s = 1 / (1 + exp(-z)) with exp(-z) = 2^(-z log2 e) and the fast

@@ -31,6 +31,8 @@ struct DevVol {
 // Parameters shared by the askAdam kernels (passed by value).
 struct AdamParams {
     DevProtocol P;
+    NexiNodes nodes;
+    int node_smem;         // the launch has room for the node table in shared memory
     int nm, np, nvtot;            // nvtot: padded voxel count, array stride
     const float* data;            // [nm][nvtot]
     const float* weights;         // [nm][nvtot] or nullptr
@@ -165,6 +167,8 @@ cudaError_t launch_forward_only(const DevProtocol& P, int model, const float* th
 // MCMC (mcmc_kernels.cu).
 struct McmcParams {
     DevProtocol P;
+    NexiNodes nodes;
+    int node_smem;         // the launch has room for the node table in shared memory
     int nm, nvar, nvox;
     const float* data;     // [nm][nvox]
     const float* weights;  // [nm][nvox] or nullptr
@@ -202,6 +206,10 @@ cudaError_t launch_mcmc_partners(const McmcParams& p, int* partner, cudaStream_t
 // goodman_weare_wglobal_constant launch shape: voxels per CTA, threads, CTAs
 // (= rows of the partial-sum table) and dynamic shared memory.
 void gwg_launch_shape(const McmcParams& p, int block_hint, int* vpb, int* block, int* nblocks, size_t* smem);
+// Node table of a NEXI protocol (capi.cu); its place in dynamic shared memory.
+constexpr size_t kMaxSmemPerBlock = 227 * 1024;
+void make_nodes(const DevProtocol& P, NexiNodes* t);
+int nodes_fit(size_t* smem);
 cudaError_t launch_mcmc(const McmcParams& p, int model, int block, cudaStream_t s);
 // Launch shapes the MCMC autotuner tries (threads per block), and one trial
 // launch of steps 1..k1 from the start into scratch state and sums.

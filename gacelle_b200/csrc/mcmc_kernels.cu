@@ -149,6 +149,13 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
     if (MODEL == kR1R2S)
         for (int f = 0; f < p.P.n_fa; ++f) sincosf(b1 * p.P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
+    if constexpr (kIsNexi<MODEL>)
+        if (p.node_smem) {  // behind the rest, at a 16-byte boundary
+            NexiNodes* s_nodes = reinterpret_cast<NexiNodes*>(
+                smem_raw + ((sizeof(double) * 2 * vpb * W * NV + sizeof(float) * (vpb * W * NV + 2 * vpb * nm) + 15) & ~(size_t)15));
+            stage_nodes(p.nodes, s_nodes);
+            va.nodes = s_nodes;
+        }
 
     // walkers owned by this thread: slot 0 (simultaneous: walker a; red-black:
     // walker a of the first half, if any) and, red-black, slot 1 (walker h + a)
@@ -298,6 +305,8 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
                           double* lpstate, double* sum, double* sumsq) {
     __shared__ DevProtocol s_P;
     stage_protocol(p.P, &s_P);
+    __shared__ __align__(16) unsigned char s_nodes[kIsNexi<MODEL> ? sizeof(NexiNodes) : 16];
+    if constexpr (kIsNexi<MODEL>) stage_nodes(p.nodes, reinterpret_cast<NexiNodes*>(s_nodes));
     __syncthreads();
     int v = blockIdx.x * blockDim.x + threadIdx.x;
     bool live = v < p.nvox;
@@ -309,6 +318,7 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
     if (MODEL == kR1R2S)
         for (int f = 0; f < p.P.n_fa; ++f) sincosf(b1 * p.P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
+    if constexpr (kIsNexi<MODEL>) va.nodes = reinterpret_cast<const NexiNodes*>(s_nodes);
     float x[NV];
     double lp = 0.0;
     double s1[NV], s2[NV];
@@ -472,6 +482,14 @@ __global__ void gwg_step_kernel(McmcParams p, int rr, int k, int warm, int flags
     if (MODEL == kR1R2S)
         for (int f = 0; f < p.P.n_fa; ++f) sincosf(b1 * p.P.fa_rad[f], &sa[f], &ca[f]);
     VoxAux va{b1, sa, ca, 1};
+    if constexpr (kIsNexi<MODEL>)
+        if (p.node_smem) {
+            NexiNodes* s_nodes = reinterpret_cast<NexiNodes*>(
+                smem_raw + ((sizeof(double) * vpb * W + sizeof(float) * (vpb * W * nvar + 2 * W * nvar + 2 * vpb * nm) + 15) &
+                            ~(size_t)15));
+            stage_nodes(p.nodes, s_nodes);
+            va.nodes = s_nodes;
+        }
     float x[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) x[q] = 0.0f;
@@ -742,7 +760,7 @@ static void gw_shape(const McmcParams& p, int block_hint, int* vpb, int* block, 
 
 // Steps [k0, k1] of repetition rr as one launch (init: the walkers start at k0 == 1).
 template <int MODEL>
-static cudaError_t mcmc_launch_steps(const McmcParams& p, int block_hint, int rr, int k0, int k1, float* xstate,
+static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k0, int k1, float* xstate,
                                      double* lpstate, double* sum, double* sumsq, cudaStream_t s) {
     constexpr int NV = ModelNP<MODEL>::value + 1;  // the model's parameters and the noise sigma
     if (p.nvar != NV) return cudaErrorInvalidValue;
@@ -752,7 +770,8 @@ static cudaError_t mcmc_launch_steps(const McmcParams& p, int block_hint, int rr
         gw_shape(p, block_hint, &vpb, &block, &smem);
         const int nb = (p.nvox + vpb - 1) / vpb;
         auto k = p.update == 0 ? gw_kernel<MODEL, NV, false> : gw_kernel<MODEL, NV, true>;
-        if (smem > 48 * 1024) {
+        if (kIsNexi<MODEL>) p.node_smem = nodes_fit(&smem);
+        if (smem + sizeof(DevProtocol) > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
         }
@@ -824,13 +843,14 @@ void gwg_launch_shape(const McmcParams& p, int block_hint, int* vpb, int* block,
 }
 
 template <int MODEL>
-static cudaError_t mcmc_run_global(const McmcParams& p, int block_hint, cudaStream_t s, float* xstate,
+static cudaError_t mcmc_run_global(McmcParams p, int block_hint, cudaStream_t s, float* xstate,
                                    double* lpstate) {
     if (p.nvar != ModelNP<MODEL>::value + 1) return cudaErrorInvalidValue;
     int vpb, block, nb;
     size_t smem;
     gwg_launch_shape(p, block_hint, &vpb, &block, &nb, &smem);
-    if (smem > 48 * 1024) {
+    if (kIsNexi<MODEL>) p.node_smem = nodes_fit(&smem);
+    if (smem + sizeof(DevProtocol) > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(gwg_step_kernel<MODEL, ModelNP<MODEL>::value + 1>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

@@ -199,6 +199,7 @@ extern "C" gx_status gx_askadam_noalloc(const gx_model* model, const float* data
     AdamParams a;
     memset(&a, 0, sizeof(a));
     a.P = P;
+    make_nodes(P, &a.nodes);
     a.nm = nm;
     a.np = np;
     a.nvtot = (int)nvtot;

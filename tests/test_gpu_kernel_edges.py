@@ -51,3 +51,19 @@ def test_nexi_node_table_and_loop(ctx, kind, nx):
     assert abs(loss.value - Lo) <= 1e-5 * abs(Lo) + 1e-7
     for k in range(th.shape[0]):
         assert np.max(np.abs(g[k] - go[k])) <= 1e-3 * np.max(np.abs(go[k])) + 1e-12
+
+
+@pytest.mark.parametrize("n_te", [20, 22, 23, 24])
+def test_block_near_the_default_shared_memory_limit(ctx, n_te):
+    """A 512-thread block whose measurements and staged protocol lie around
+    48 KB together runs, and fits what a 128-thread block fits (each voxel's
+    arithmetic does not depend on the block)."""
+    from helpers import run_engine
+    rng = np.random.default_rng(n_te)
+    te = np.linspace(2e-3, 40e-3, n_te)
+    th = np.vstack([rng.uniform(0.5, 1.5, 700), rng.uniform(10, 60, 700)])
+    y = th[0] * np.exp(-te[:, None] * th[1]) + 0.01 * rng.standard_normal((n_te, 700))
+    th0 = np.tile(np.array([[1.0], [30.0]], np.float32), (1, 700))
+    a, b = (run_engine("r2s", y, th0, fitting(iteration=20, blockSize=n), NAMES["r2s"], context=ctx, te=te)
+            for n in (512, 128))
+    assert np.array_equal(a["final_theta"], b["final_theta"])
