@@ -91,7 +91,7 @@ enum Slot {
     S_MC_PART, S_MC_SUM, S_MC_SUMSQ, S_MC_SHIFT, S_MC_X0, S_MC_POST, S_MC_ACC, S_MC_MEAN,
     S_MC_STD, S_FWD_TH, S_FWD_SIG, S_FWD_B1, S_BAR, S_MC_GLOB, S_ROBUST, S_DICT_SIG, S_DICT_D,
     S_DICT_W, S_DICT_E, S_DICT_C, S_DICT_B, S_DICT_S, S_FLAGS, S_DATA_QUADS, S_PRIOR_MU, S_PRIOR_SD, S_SURF_NB, S_SURF_LEN,
-    S_MC_STATS, S_TUNE, S_TUNE_HIST, S_BLK_L, S_HGRID0, S_HGRID1, S_NSLOTS
+    S_MC_STATS, S_MC_X, S_MC_LP, S_TUNE, S_TUNE_HIST, S_BLK_L, S_HGRID0, S_HGRID1, S_NSLOTS
 };
 
 struct gx_context {
@@ -1644,7 +1644,8 @@ static gx_status tune_mcmc(gx_context* c, const McmcParams& p, int model, int* b
         McmcParams t = p;
         t.nvox = std::min(p.nvox, std::max(256, (1 << 19) / W));
         t.posterior = nullptr;
-        const int k1 = std::min(p.iteration, 8);
+        // MH steps are short: enough of them to tell the blocks apart
+        const int k1 = std::min(p.iteration, p.algorithm == 1 ? 8 : 64);
         const size_t nx = (size_t)t.nvar * t.nvox * W, nl = (size_t)t.nvox * W, ns = (size_t)t.nvar * t.nvox;
         const size_t o_lp = (sizeof(float) * nx + 255) / 256 * 256;
         const size_t o_s1 = o_lp + (sizeof(double) * nl + 255) / 256 * 256;
@@ -1827,12 +1828,16 @@ extern "C" gx_status gx_mcmc(gx_context* c, const gx_model* model, int32_t mem, 
         int block = o->block_size;
         if (block == 0 && ng == 0 && autotune_enabled()) TRY(tune_mcmc(c, p, id, &block, &tuned_now));
         block_used = block > 0 ? block : 128;
+        float* xstate;
+        double* lpstate;
+        TRY(wsT(c, S_MC_X, (size_t)nvar * nv * W, &xstate));
+        TRY(wsT(c, S_MC_LP, (size_t)nv * W, &lpstate));
         CK(cudaEventRecord(c->ev[2], c->stream));
-        CK(launch_mcmc(p, id, block, c->stream));
+        CK(launch_mcmc(p, id, block, xstate, lpstate, c->stream));
         CK(cudaEventRecord(c->ev[3], c->stream));
         launches += ng > 0 ? (o->ensemble_update == GX_GW_REDBLACK ? 4 : 2) * (o->iteration + o->global_warmup) *
                                  o->repetition
-                           : (o->iteration + 249) / 250 * o->repetition;
+                           : (o->iteration - 1) / mcmc_steps_per_launch(p) * o->repetition + o->repetition;
         float *mean = nullptr, *stdv = nullptr;
         if (mem == GX_MEM_DEVICE) { mean = r.mean; stdv = r.std; }
         else {

@@ -206,11 +206,13 @@ cudaError_t launch_mcmc_partners(const McmcParams& p, int* partner, cudaStream_t
 // goodman_weare_wglobal_constant launch shape: voxels per CTA, threads, CTAs
 // (= rows of the partial-sum table) and dynamic shared memory.
 void gwg_launch_shape(const McmcParams& p, int block_hint, int* vpb, int* block, int* nblocks, size_t* smem);
+int mcmc_steps_per_launch(const McmcParams& p);
 // Node table of a NEXI protocol (capi.cu); its place in dynamic shared memory.
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
 void make_nodes(const DevProtocol& P, NexiNodes* t);
 int nodes_fit(size_t* smem);
-cudaError_t launch_mcmc(const McmcParams& p, int model, int block, cudaStream_t s);
+// xstate [nvar][nvox][W], lpstate [nvox][W] (W = 1 for MH): the walkers between launches
+cudaError_t launch_mcmc(const McmcParams& p, int model, int block, float* xstate, double* lpstate, cudaStream_t s);
 // Launch shapes the MCMC autotuner tries (threads per block), and one trial
 // launch of steps 1..k1 from the start into scratch state and sums.
 int mcmc_block_candidates(const McmcParams& p, int* out, int maxn);

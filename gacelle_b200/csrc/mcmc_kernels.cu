@@ -9,6 +9,8 @@
 // written out as the full posterior).  Reference: utils/mcmc.m
 // (metropolis_hastings :82-190, goodman_weare :192-383, find_partner
 // :797-803, res2out :806-862), utils/logP_Gaussian.m.
+#include <algorithm>
+
 #include "gx_internal.h"
 
 namespace gx {
@@ -82,6 +84,80 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
     return -sink.sos / (2.0 * n2) - 0.5 * nm * log(6.283185307179586 * n2);
 }
 
+// Screened acceptance (R2*, unit weights, up to kScreenM measurements).
+//
+// The decision lr > log u needs the FP64 log-likelihoods (division, logarithm
+// and an FP64 sum: a third of a step's instructions, and its longest
+// dependent chain) only when the two sides are close.  The screen evaluates
+// both in FP32 with a bound on its error, and the FP64 form (log_prob_t, the
+// same values whenever it is evaluated) decides inside the bound, about one
+// proposal in 10^4; so every decision is the FP64 one.  With n the noise,
+// a = sos / (2 n^2) and the constant nm log(2 pi) / 2 cancelling,
+//   log p' - log p = (a - a') + nm (log n - log n').
+// Error, with e = 2^-24: the residuals are the FP64 form's (same operations);
+// the FP32 sum of their nm squares and the FP64 sum of the rounded squares
+// differ by at most (nm + 1) e relative, a by at most another 6 e (n^2,
+// reciprocal of 1 ulp, two products): (nm + 20) e.  __logf is within
+// 2^-21.4 absolute or 3 ulp relative of the logarithm, and the roundings of
+// the sums are below 2^-21 of their terms: 2^-20 of every term's magnitude
+// plus 2^-20 for every logarithm.  NaN and infinities fail both tests and go
+// to the FP64 form.  Measurements in registers, echo constants in the constant
+// bank.  12,013 voxels x 50 walkers x 500 steps, 12 echoes: 6.93 -> 4.09 ms;
+// Metropolis-Hastings, 4096 voxels x 10,000 steps: 15.4 -> 8.4 ms (one
+// dependent chain a voxel, 1.4-2.1 -> 0.8 us a step).
+constexpr int kScreenM = 16;
+
+struct Screen {
+    float a, ln;  // sos / (2 n^2), log n
+};
+
+// Residual of one echo, M0 exp(-te R2*) - y, as log_prob_t forms it.
+__device__ __forceinline__ float r2s_residual(float te_l2e, float M0, float R2, float y) {
+    return fma1(M0, ex2_ftz(mul1(-te_l2e, R2)), -y);
+}
+
+// P: the protocol in the constant bank (compile-time indices).
+__device__ __forceinline__ Screen screen_eval(const DevProtocol& P, int nm, const float (&x)[3],
+                                              const float (&y)[kScreenM]) {
+    float s = 0.0f;
+#pragma unroll
+    for (int g = 0; g < kScreenM; g += 4) {
+        if (g + 4 <= nm) {
+#pragma unroll
+            for (int m = g; m < g + 4; ++m) {
+                const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m]);
+                s = fma1(r, r, s);
+            }
+        } else {
+#pragma unroll
+            for (int m = g; m < g + 3; ++m)
+                if (m < nm) {
+                    const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m]);
+                    s = fma1(r, r, s);
+                }
+        }
+    }
+    return Screen{s * rcp_ftz(2.0f * x[2] * x[2]), __logf(x[2])};
+}
+
+// 1 accept, 0 reject, -1 undecided: cz log(zz) + (log p(n) - log p(c)) > log(u)
+__device__ __forceinline__ int screen_decide(int nm, const Screen& c, const Screen& n, float cz, float zz, float u) {
+    const float fm = (float)nm;
+    const float lz = cz * __logf(zz), lu = __logf(u);
+    const float d = ((c.a - n.a) + fm * (c.ln - n.ln)) + (lz - lu);
+    const float tol = (fm + 20.0f) * 5.9604645e-8f * (c.a + n.a) +
+                      9.536743e-7f * (fm * (2.0f + fabsf(c.ln) + fabsf(n.ln)) + fabsf(lz) + fabsf(lu) + cz + 2.0f);
+    return d > tol ? 1 : (d < -tol ? 0 : -1);
+}
+
+// Steps k with a kept sample, k > nburnin and (k - nburnin + 1) % thinning
+// == 0: the first one at or after k0 (a launch steps from it by thinning).
+__device__ __forceinline__ int first_kept(const McmcParams& p, int k0) {
+    const int k = max(k0, p.nburnin + 1);
+    const int r = (k - p.nburnin + 1) % p.thinning;
+    return r ? k + p.thinning - r : k;
+}
+
 __device__ __forceinline__ int kept_index(const McmcParams& p, int k) {
     if (k <= p.nburnin) return -1;
     int j = k - p.nburnin + 1;
@@ -115,7 +191,9 @@ __device__ __forceinline__ void gw_walker_start(const McmcParams& p, int v, int 
 // keep every per-walker vector in registers; the running sums of the kept
 // samples live in shared memory (each thread its own walkers' slots) and are
 // folded into the per-voxel sums at the end of the launch.
-template <int MODEL, int NV, bool RB>
+// SCREEN: acceptance decided by the FP32 screen where it can; the walkers'
+// log-likelihoods are then not kept (xstate determines them).
+template <int MODEL, int NV, bool RB, bool SCREEN>
 __global__ void __launch_bounds__(1024, 1)
 gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double* lpstate, double* sum,
           double* sumsq) {
@@ -163,6 +241,8 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
     const bool own0 = live && wown0 >= 0 && wown0 < W, own1 = RB && live && wown1 >= 0 && wown1 < W;
     float x0s[NV], x1s[RB ? NV : 1];
     double lp0 = 0.0, lp1 = 0.0;
+    Screen c0{0.0f, 0.0f}, c1{0.0f, 0.0f};
+    float yr[SCREEN ? kScreenM : 1];
 #pragma unroll
     for (int q = 0; q < NV; ++q) x0s[q] = 0.0f;
 #pragma unroll
@@ -193,16 +273,25 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
         }
     }
     __syncthreads();
-    if (own0) lp0 = init ? log_prob_t<MODEL, NV>(nm, s_P, x0s, yv, 1, wv, 1, va) : lpstate[(size_t)v * W + wown0];
-    if constexpr (RB)
-        if (own1) lp1 = init ? log_prob_t<MODEL, NV>(nm, s_P, x1s, yv, 1, wv, 1, va) : lpstate[(size_t)v * W + wown1];
+    if constexpr (SCREEN) {
+#pragma unroll
+        for (int m = 0; m < kScreenM; ++m) yr[m] = live && m < nm ? yv[m] : 0.0f;
+        if (own0) c0 = screen_eval(p.P, nm, x0s, yr);
+        if constexpr (RB)
+            if (own1) c1 = screen_eval(p.P, nm, x1s, yr);
+    } else {
+        if (own0) lp0 = init ? log_prob_t<MODEL, NV>(nm, s_P, x0s, yv, 1, wv, 1, va) : lpstate[(size_t)v * W + wown0];
+        if constexpr (RB)
+            if (own1) lp1 = init ? log_prob_t<MODEL, NV>(nm, s_P, x1s, yv, 1, wv, 1, va) : lpstate[(size_t)v * W + wown1];
+    }
     unsigned int nacc = 0;
     const float amin1 = p.a - 1.0f;
+    int kept_k = first_kept(p, k0);
 
     // stretch proposal of walker w (state xw, log-likelihood lpw) about its
     // partner: xn and its log-likelihood lpp, and whether it is accepted
-    auto propose = [&](int w, int k, uint32_t flags, const float (&xw)[NV], double lpw, float (&xn)[NV],
-                       double& lpp) -> bool {
+    auto propose = [&](int w, int k, uint32_t flags, const float (&xw)[NV], double lpw, const Screen& cw,
+                       float (&xn)[NV], double& lpp, Screen& cn) -> bool {
         const int* pt = p.partner + ((size_t)rr * p.iteration + (k - 1)) * W;
         const int q = pt[w];
         U4 u = philox((uint32_t)v, (uint32_t)w, (uint32_t)k, kTagGwMove | ((uint32_t)rr << 16) | flags, p.seed);
@@ -216,17 +305,30 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
             oob |= (xp < p.lb[j]) || (xp > p.ub[j]);
             xn[j] = fminf(fmaxf(xp, p.lb[j]), p.ub[j]);
         }
+        if constexpr (SCREEN) {
+            cn = screen_eval(p.P, nm, xn, yr);
+            int d = screen_decide(nm, cw, cn, (float)(NV - 1), zz, u01(u.y));
+            if (d < 0 && !oob) {
+                const double lr = (double)(NV - 1) * (double)logf(zz) +
+                                  (log_prob_t<MODEL, NV>(nm, s_P, xn, yv, 1, wv, 1, va) -
+                                   log_prob_t<MODEL, NV>(nm, s_P, xw, yv, 1, wv, 1, va));
+                d = lr > (double)logf(u01(u.y));
+            }
+            return !oob && d > 0;
+        }
         lpp = log_prob_t<MODEL, NV>(nm, s_P, xn, yv, 1, wv, 1, va);
         double lr = (double)(NV - 1) * (double)logf(zz) + (lpp - lpw);
         return !oob && lr > (double)logf(u01(u.y));
     };
-    auto commit = [&](int w, const float (&xn)[NV], double lpp, float (&xw)[NV], double& lpw) {
+    auto commit = [&](int w, const float (&xn)[NV], double lpp, const Screen& cn, float (&xw)[NV], double& lpw,
+                      Screen& cw) {
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             xw[j] = xn[j];
             xv[w * NV + j] = xn[j];
         }
-        lpw = lpp;
+        if constexpr (SCREEN) cw = cn;
+        else lpw = lpp;
         ++nacc;
     };
     auto keep = [&](int w, int c, const float (&xw)[NV]) {
@@ -244,43 +346,49 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
         if constexpr (!RB) {
             float xn[NV];
             double lpp = 0.0;
-            const bool acc = own0 && propose(wown0, k, 0u, x0s, lp0, xn, lpp);
+            Screen cn{0.0f, 0.0f};
+            const bool acc = own0 && propose(wown0, k, 0u, x0s, lp0, c0, xn, lpp, cn);
             __syncthreads();  // every walker has read the old ensemble
-            if (acc) commit(wown0, xn, lpp, x0s, lp0);
+            if (acc) commit(wown0, xn, lpp, cn, x0s, lp0, c0);
             __syncthreads();
         } else {
             // the active half moves about anchors in the frozen half
             if (own0) {
                 float xn[NV];
                 double lpp = 0.0;
-                if (propose(wown0, k, 1u << 8, x0s, lp0, xn, lpp)) commit(wown0, xn, lpp, x0s, lp0);
+                Screen cn{0.0f, 0.0f};
+                if (propose(wown0, k, 1u << 8, x0s, lp0, c0, xn, lpp, cn)) commit(wown0, xn, lpp, cn, x0s, lp0, c0);
             }
             __syncthreads();  // the moved half is visible before the other half anchors on it
             if (own1) {
                 float xn[NV];
                 double lpp = 0.0;
-                if (propose(wown1, k, 1u << 8, x1s, lp1, xn, lpp)) commit(wown1, xn, lpp, x1s, lp1);
+                Screen cn{0.0f, 0.0f};
+                if (propose(wown1, k, 1u << 8, x1s, lp1, c1, xn, lpp, cn)) commit(wown1, xn, lpp, cn, x1s, lp1, c1);
             }
             __syncthreads();
         }
-        const int c = kept_index(p, k);
-        if (c >= 0) {
-            if (own0) keep(wown0, c, x0s);
-            if constexpr (RB)
-                if (own1) keep(wown1, c, x1s);
+        if (k == kept_k) {
+            kept_k += p.thinning;
+            const int c = kept_index(p, k);
+            if (c >= 0) {
+                if (own0) keep(wown0, c, x0s);
+                if constexpr (RB)
+                    if (own1) keep(wown1, c, x1s);
+            }
         }
     }
     // persist walker state, fold the kept-sample sums of this launch
     if (own0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) xstate[((size_t)q * p.nvox + v) * W + wown0] = x0s[q];
-        lpstate[(size_t)v * W + wown0] = lp0;
+        if constexpr (!SCREEN) lpstate[(size_t)v * W + wown0] = lp0;
     }
     if constexpr (RB) {
         if (own1) {
 #pragma unroll
             for (int q = 0; q < NV; ++q) xstate[((size_t)q * p.nvox + v) * W + wown1] = x1s[q];
-            lpstate[(size_t)v * W + wown1] = lp1;
+            if constexpr (!SCREEN) lpstate[(size_t)v * W + wown1] = lp1;
         }
     }
     if (live) {
@@ -299,8 +407,12 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
 
 // Metropolis-Hastings, one thread per voxel (mcmc.m:144-167).  NV =
 // parameters + noise at compile time (the state in registers); the voxel's
-// measurements are read from [nm][nvox] with coalesced loads.
-template <int MODEL, int NV>
+// measurements are read from [nm][nvox] with coalesced loads, once into
+// registers when the acceptance is screened (SCREEN).  A step's draws do not
+// depend on the state, so those of step k + 1 are made while step k's
+// proposal is evaluated: with few voxels a step is one dependent chain, and
+// the draws fill its latencies.
+template <int MODEL, int NV, bool SCREEN>
 __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate,
                           double* lpstate, double* sum, double* sumsq) {
     __shared__ DevProtocol s_P;
@@ -321,31 +433,44 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
     if constexpr (kIsNexi<MODEL>) va.nodes = reinterpret_cast<const NexiNodes*>(s_nodes);
     float x[NV];
     double lp = 0.0;
+    Screen cs{0.0f, 0.0f};
+    float yr[SCREEN ? kScreenM : 1];
     double s1[NV], s2[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) { s1[q] = 0.0; s2[q] = 0.0; x[q] = 0.0f; }
     unsigned int nacc = 0;
+    // the draws of step k: normals for the proposal and the acceptance uniform
+    constexpr int ND = (NV + 3) / 4 * 4;
+    auto draws = [&](int k, float (&nrm)[ND], float& u) {
+        const uint32_t tag = kTagMhMove | ((uint32_t)rr << 16);
+#pragma unroll
+        for (int j = 0; j * 4 < NV; ++j) {
+            U4 r = philox((uint32_t)v, (uint32_t)k, (uint32_t)j, tag, p.seed);
+            box_muller(r.x, r.y, nrm[4 * j], nrm[4 * j + 1]);
+            box_muller(r.z, r.w, nrm[4 * j + 2], nrm[4 * j + 3]);
+        }
+        u = u01(philox((uint32_t)v, (uint32_t)k, 8u, tag, p.seed).x);
+    };
     if (live) {
         if (init) {
 #pragma unroll
             for (int q = 0; q < NV; ++q)
                 x[q] = fminf(fmaxf(p.x0[(size_t)q * p.nvox + v], p.lb[q]), p.ub[q]);
-            lp = log_prob_t<MODEL, NV>(nm, s_P, x, yv, p.nvox, wv, p.nvox, va);
+            if constexpr (!SCREEN) lp = log_prob_t<MODEL, NV>(nm, s_P, x, yv, p.nvox, wv, p.nvox, va);
         } else {
 #pragma unroll
             for (int q = 0; q < NV; ++q) x[q] = xstate[(size_t)q * p.nvox + v];
-            lp = lpstate[v];
+            if constexpr (!SCREEN) lp = lpstate[v];
         }
-        for (int k = k0; k <= k1; ++k) {
-            float nrm[(NV + 3) / 4 * 4];
-            uint32_t tag = kTagMhMove | ((uint32_t)rr << 16);
+        if constexpr (SCREEN) {
 #pragma unroll
-            for (int j = 0; j * 4 < NV; ++j) {
-                U4 u = philox((uint32_t)v, (uint32_t)k, (uint32_t)j, tag, p.seed);
-                box_muller(u.x, u.y, nrm[4 * j], nrm[4 * j + 1]);
-                box_muller(u.z, u.w, nrm[4 * j + 2], nrm[4 * j + 3]);
-            }
-            U4 ua = philox((uint32_t)v, (uint32_t)k, 8u, tag, p.seed);
+            for (int m = 0; m < kScreenM; ++m) yr[m] = m < nm ? yv[(size_t)m * p.nvox] : 0.0f;
+            cs = screen_eval(p.P, nm, x, yr);
+        }
+        int kept_k = first_kept(p, k0);
+        float nrm[ND], u;
+        draws(k0, nrm, u);
+        for (int k = k0; k <= k1; ++k) {
             float xp[NV];
             bool oob = false;
 #pragma unroll
@@ -354,27 +479,45 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
                 oob |= (t < p.lb[q]) || (t > p.ub[q]);
                 xp[q] = fminf(fmaxf(t, p.lb[q]), p.ub[q]);
             }
-            double lpp = log_prob_t<MODEL, NV>(nm, s_P, xp, yv, p.nvox, wv, p.nvox, va);
-            if (!oob && (lpp - lp) > (double)logf(u01(ua.x))) {
+            const float uk = u;
+            bool acc;
+            if constexpr (SCREEN) {
+                const Screen cp = screen_eval(p.P, nm, xp, yr);
+                draws(k + 1, nrm, u);
+                int d = screen_decide(nm, cs, cp, 0.0f, 1.0f, uk);
+                if (d < 0 && !oob)
+                    d = (log_prob_t<MODEL, NV>(nm, s_P, xp, yv, p.nvox, wv, p.nvox, va) -
+                         log_prob_t<MODEL, NV>(nm, s_P, x, yv, p.nvox, wv, p.nvox, va)) > (double)logf(uk);
+                acc = !oob && d > 0;
+                if (acc) cs = cp;
+            } else {
+                const double lpp = log_prob_t<MODEL, NV>(nm, s_P, xp, yv, p.nvox, wv, p.nvox, va);
+                draws(k + 1, nrm, u);
+                acc = !oob && (lpp - lp) > (double)logf(uk);
+                if (acc) lp = lpp;
+            }
+            if (acc) {
 #pragma unroll
                 for (int q = 0; q < NV; ++q) x[q] = xp[q];
-                lp = lpp;
                 ++nacc;
             }
-            int c = kept_index(p, k);
-            if (c >= 0)
+            if (k == kept_k) {
+                kept_k += p.thinning;
+                const int c = kept_index(p, k);
+                if (c >= 0)
 #pragma unroll
-                for (int j = 0; j < NV; ++j) {
-                    double d = (double)x[j] - (double)p.shift[(size_t)j * p.nvox + v];
-                    s1[j] += d;
-                    s2[j] += d * d;
-                    if (p.posterior)
-                        p.posterior[(((size_t)j * p.repetition + rr) * p.ns + c) * p.nvox + v] = x[j];
-                }
+                    for (int j = 0; j < NV; ++j) {
+                        double d = (double)x[j] - (double)p.shift[(size_t)j * p.nvox + v];
+                        s1[j] += d;
+                        s2[j] += d * d;
+                        if (p.posterior)
+                            p.posterior[(((size_t)j * p.repetition + rr) * p.ns + c) * p.nvox + v] = x[j];
+                    }
+            }
         }
 #pragma unroll
         for (int q = 0; q < NV; ++q) xstate[(size_t)q * p.nvox + v] = x[q];
-        lpstate[v] = lp;
+        if constexpr (!SCREEN) lpstate[v] = lp;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             sum[(size_t)j * p.nvox + v] += s1[j];
@@ -758,6 +901,10 @@ static void gw_shape(const McmcParams& p, int block_hint, int* vpb, int* block, 
             sizeof(float) * ((size_t)(*vpb) * W * p.nvar + 2 * (size_t)(*vpb) * p.nm);
 }
 
+// The screen's bound holds for a sum of squares (no weights), and its
+// measurements are held in registers.
+static bool screened(const McmcParams& p) { return p.weights == nullptr && p.nm <= kScreenM; }
+
 // Steps [k0, k1] of repetition rr as one launch (init: the walkers start at k0 == 1).
 template <int MODEL>
 static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k0, int k1, float* xstate,
@@ -769,7 +916,9 @@ static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k
         size_t smem;
         gw_shape(p, block_hint, &vpb, &block, &smem);
         const int nb = (p.nvox + vpb - 1) / vpb;
-        auto k = p.update == 0 ? gw_kernel<MODEL, NV, false> : gw_kernel<MODEL, NV, true>;
+        auto k = p.update == 0 ? gw_kernel<MODEL, NV, false, false> : gw_kernel<MODEL, NV, true, false>;
+        if constexpr (MODEL == kR2S)
+            if (screened(p)) k = p.update == 0 ? gw_kernel<MODEL, NV, false, true> : gw_kernel<MODEL, NV, true, true>;
         if (kIsNexi<MODEL>) p.node_smem = nodes_fit(&smem);
         if (smem + sizeof(DevProtocol) > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -779,16 +928,27 @@ static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k
     } else {
         const int block = block_hint > 0 ? block_hint : 128;
         const int nb = (p.nvox + block - 1) / block;
-        mh_kernel<MODEL, NV><<<nb, block, 0, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, lpstate, sum, sumsq);
+        auto k = mh_kernel<MODEL, NV, false>;
+        if constexpr (MODEL == kR2S)
+            if (screened(p)) k = mh_kernel<MODEL, NV, true>;
+        k<<<nb, block, 0, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, lpstate, sum, sumsq);
     }
     ++g_kernel_launches;
     return cudaGetLastError();
 }
 
+// Steps per launch: a bounded kernel duration (below a second for a million
+// walkers), and enough steps that few walkers do not spend their time on
+// launches, each of which reloads the state.
+int mcmc_steps_per_launch(const McmcParams& p) {
+    const size_t walkers = (size_t)p.nvox * (p.algorithm == 1 ? p.nwalker : 1);
+    return (int)std::min<size_t>(5000, std::max<size_t>(250, 250000000 / walkers));
+}
+
 template <int MODEL>
 static cudaError_t mcmc_run_model(const McmcParams& p, int block_hint, cudaStream_t s,
                                   float* xstate, double* lpstate) {
-    const int chunk = 250;  // steps per launch: bounded kernel duration
+    const int chunk = mcmc_steps_per_launch(p);
     for (int rr = 0; rr < p.repetition; ++rr)
         for (int k0 = 1; k0 <= p.iteration; k0 += chunk) {
             int k1 = k0 + chunk - 1 < p.iteration ? k0 + chunk - 1 : p.iteration;
@@ -809,7 +969,7 @@ int mcmc_block_candidates(const McmcParams& p, int* out, int maxn) {
             out[n++] = block;
         }
     } else {
-        for (int b = 64; b <= 512 && n < maxn; b *= 2) out[n++] = b;
+        for (int b = 32; b <= 512 && n < maxn; b *= 2) out[n++] = b;
     }
     return n;
 }
@@ -901,37 +1061,23 @@ static cudaError_t mcmc_run_global(McmcParams p, int block_hint, cudaStream_t s,
     return cudaGetLastError();
 }
 
-cudaError_t launch_mcmc(const McmcParams& p, int model, int block, cudaStream_t s) {
-    // walker state between chunked launches
-    size_t W = p.algorithm == 1 ? (size_t)p.nwalker : 1;
-    float* xstate = nullptr;
-    double* lpstate = nullptr;
-    cudaError_t e = cudaMallocAsync(&xstate, sizeof(float) * p.nvar * p.nvox * W, s);
-    if (e != cudaSuccess) return e;
-    e = cudaMallocAsync(&lpstate, sizeof(double) * p.nvox * W, s);
-    if (e != cudaSuccess) { cudaFreeAsync(xstate, s); return e; }
+cudaError_t launch_mcmc(const McmcParams& p, int model, int block, float* xstate, double* lpstate, cudaStream_t s) {
     mcmc_shift_kernel<<<(p.nvox + 127) / 128, 128, 0, s>>>(p);
     ++g_kernel_launches;
     if (p.ng > 0) {
         switch (model) {
-        case kR2S: e = mcmc_run_global<kR2S>(p, block, s, xstate, lpstate); break;
-        case kR1R2S: e = mcmc_run_global<kR1R2S>(p, block, s, xstate, lpstate); break;
-        case kNEXI: e = mcmc_run_global<kNEXI>(p, block, s, xstate, lpstate); break;
-        default: e = mcmc_run_global<kNEXI2>(p, block, s, xstate, lpstate); break;
+        case kR2S: return mcmc_run_global<kR2S>(p, block, s, xstate, lpstate);
+        case kR1R2S: return mcmc_run_global<kR1R2S>(p, block, s, xstate, lpstate);
+        case kNEXI: return mcmc_run_global<kNEXI>(p, block, s, xstate, lpstate);
+        default: return mcmc_run_global<kNEXI2>(p, block, s, xstate, lpstate);
         }
-        cudaFreeAsync(xstate, s);
-        cudaFreeAsync(lpstate, s);
-        return e;
     }
     switch (model) {
-    case kR2S: e = mcmc_run_model<kR2S>(p, block, s, xstate, lpstate); break;
-    case kR1R2S: e = mcmc_run_model<kR1R2S>(p, block, s, xstate, lpstate); break;
-    case kNEXI: e = mcmc_run_model<kNEXI>(p, block, s, xstate, lpstate); break;
-    default: e = mcmc_run_model<kNEXI2>(p, block, s, xstate, lpstate); break;
+    case kR2S: return mcmc_run_model<kR2S>(p, block, s, xstate, lpstate);
+    case kR1R2S: return mcmc_run_model<kR1R2S>(p, block, s, xstate, lpstate);
+    case kNEXI: return mcmc_run_model<kNEXI>(p, block, s, xstate, lpstate);
+    default: return mcmc_run_model<kNEXI2>(p, block, s, xstate, lpstate);
     }
-    cudaFreeAsync(xstate, s);
-    cudaFreeAsync(lpstate, s);
-    return e;
 }
 
 int mcmc_missing_slots(const McmcParams& p) {

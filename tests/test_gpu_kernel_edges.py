@@ -53,6 +53,38 @@ def test_nexi_node_table_and_loop(ctx, kind, nx):
         assert np.max(np.abs(g[k] - go[k])) <= 1e-3 * np.max(np.abs(go[k])) + 1e-12
 
 
+def _r2s_chain(ctx, te, update, nv, W, steps, weights=None, **over):
+    from gacelle_b200 import mcmc_solver
+    from gacelle_b200.models import gpuR2starMapping
+    rng = np.random.default_rng(len(te))
+    m = gpuR2starMapping(te)
+    th = np.vstack([rng.uniform(0.5, 1.5, nv), rng.uniform(10, 60, nv)])
+    y = (th[0] * np.exp(-te[:, None] * th[1]) + 0.02 * rng.standard_normal((len(te), nv))).astype(np.float32)
+    x0 = np.vstack([th, np.full(nv, 0.02)]).astype(np.float32)
+    f = mcmc_solver.check_set_default_basic(dict({
+        "algorithm": "MH" if update == "mh" else "GW", "iteration": steps, "thinning": 1, "burnin": 0.0,
+        "Nwalker": W, "Ensembleupdate": "redblack" if update == "redblack" else "simultaneous", "lb": m.lb,
+        "ub": m.ub, "xStepSize": m.step, "seed": 9}, **over))
+    eng = mcmc_solver.mcmc(ctx)._run(m, y, weights, x0, None, m.modelParams, f, True)
+    ref = oracle.mcmc(oracle.r2s(te), oracle.Volume(y.astype(np.float64)), x0.astype(np.float64), m.lb, m.ub,
+                      algorithm="MH" if update == "mh" else "ensemble", iteration=steps, thinning=1, burnin=0.0, nwalker=W,
+                      seed=9, x_step=m.step, ensemble_update=f["Ensembleupdate"], want_posterior=True)
+    return eng["posterior"], ref["posterior"]
+
+
+@pytest.mark.parametrize("update", ["simultaneous", "redblack", "mh"])
+@pytest.mark.parametrize("n_te", [1, 3, 5, 12, 16, 17])
+def test_r2s_chain_decisions(ctx, update, n_te):
+    """Chains of the screened acceptance (up to 16 echoes) and of the FP64 one
+    (17) take the oracle's moves: same draws, so the samples coincide except
+    where the signal's FP32 rounding flips a decision (the bar of the sampler
+    parity tests, > 97 % over the first steps)."""
+    te = np.linspace(2e-3, 40e-3, n_te) if n_te > 1 else np.array([5e-3])
+    pe, po = _r2s_chain(ctx, te, update, 33, 1 if update == "mh" else 50, 12)
+    assert pe.shape == po.shape
+    assert np.mean(np.abs(pe - po) <= 1e-4 * np.abs(po) + 1e-7) > 0.97
+
+
 @pytest.mark.parametrize("n_te", [20, 22, 23, 24])
 def test_block_near_the_default_shared_memory_limit(ctx, n_te):
     """A 512-thread block whose measurements and staged protocol lie around
