@@ -90,7 +90,7 @@ enum Slot {
     S_GRID1, S_P_TH, S_P_DTH, S_P_SIG, S_P_DSIG, S_P_RES, S_P_GTH, S_P_GZ, S_P_ACC, S_ZMIN,
     S_MC_PART, S_MC_SUM, S_MC_SUMSQ, S_MC_SHIFT, S_MC_X0, S_MC_POST, S_MC_ACC, S_MC_MEAN,
     S_MC_STD, S_FWD_TH, S_FWD_SIG, S_FWD_B1, S_BAR, S_MC_GLOB, S_ROBUST, S_DICT_SIG, S_DICT_D,
-    S_DICT_W, S_DICT_E, S_DICT_C, S_DICT_B, S_DICT_S, S_FLAGS, S_DATA_QUADS, S_PRIOR_MU, S_PRIOR_SD, S_SURF_NB, S_SURF_LEN,
+    S_DICT_W, S_DICT_OP, S_DICT_LIST, S_DICT_STAT, S_DICT_E, S_DICT_C, S_DICT_B, S_DICT_S, S_FLAGS, S_DATA_QUADS, S_PRIOR_MU, S_PRIOR_SD, S_SURF_NB, S_SURF_LEN,
     S_MC_STATS, S_MC_X, S_MC_LP, S_TUNE, S_TUNE_HIST, S_BLK_L, S_HGRID0, S_HGRID1, S_NSLOTS
 };
 
@@ -1952,8 +1952,16 @@ extern "C" gx_status gx_dictionary_match(gx_context* c, int32_t mem, const float
     double *ie, *cj;
     TRY(wsT(c, S_DICT_E, (size_t)ndict, &ie));
     TRY(wsT(c, S_DICT_C, (size_t)ndict, &cj));
+    unsigned char* op = nullptr;
+    int* list = nullptr;
+    DictStat* stat = nullptr;
+    if (dict_tensor_ok(ndict, nm, wt != nullptr)) {
+        TRY(wsT(c, S_DICT_OP, dict_operand_bytes(ndict, nm), &op));
+        TRY(wsT(c, S_DICT_LIST, (size_t)nvox, &list));
+        TRY(wsT(c, S_DICT_STAT, 1, &stat));
+    }
     CK(cudaEventRecord(c->ev[2], c->stream));
-    CK(launch_dictionary_match(ds, nvox, dd, ndict, nm, dw, ie, cj, db, dsse, c->stream));
+    CK(launch_dictionary_match(ds, nvox, dd, ndict, nm, dw, ie, cj, db, dsse, op, list, stat, c->stream));
     CK(cudaEventRecord(c->ev[3], c->stream));
     if (mem == GX_MEM_HOST) {
         CK(cudaMemcpyAsync(best, db, sizeof(int32_t) * nvox, cudaMemcpyDeviceToHost, c->stream));
@@ -1963,7 +1971,10 @@ extern "C" gx_status gx_dictionary_match(gx_context* c, int32_t mem, const float
             d2h += sizeof(float) * nvox;
         }
     }
+    DictStat hs{};
+    if (stat) CK(cudaMemcpyAsync(&hs, stat, sizeof(hs), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (hs.err) return fail(GX_ETIMEOUT, "dictionary match: a wait expired");
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]);
     c->timing.total_ms = ms;

@@ -155,10 +155,20 @@ cudaError_t launch_robust_window(const AdamParams& a, const PlainBufs& b, int bl
 cudaError_t launch_robust_conv(const AdamParams& a, const PlainBufs& b, int block, int nblocks, cudaStream_t s);
 
 // Dictionary matching (dictionary.cu): invE, Cj are [ndict] double scratch.
+// op (dict_operand_bytes), list [nvox] and stat: scratch of the tensor-core
+// kernel where dict_tensor_ok, nullptr otherwise.
+struct DictStat {
+    int first;   // ndict minus the first entry with a positive, finite norm (0: none)
+    int n_left;  // voxels in list: left to the FP64 kernel
+    int err;     // a bounded wait expired
+    int pad;
+};
 size_t dict_match_smem(int nm, bool weighted);
+bool dict_tensor_ok(int ndict, int nm, bool weighted);
+size_t dict_operand_bytes(int ndict, int nm);
 cudaError_t launch_dictionary_match(const float* signals, int nvox, const float* dict, int ndict, int nm,
                                     const float* wt, double* invE, double* Cj, int* best, float* best_sse,
-                                    cudaStream_t s);
+                                    unsigned char* op, int* list, DictStat* stat, cudaStream_t s);
 
 // Forward only (gx_forward).
 cudaError_t launch_forward_only(const DevProtocol& P, int model, const float* theta,

@@ -99,3 +99,67 @@ def test_block_near_the_default_shared_memory_limit(ctx, n_te):
     a, b = (run_engine("r2s", y, th0, fitting(iteration=20, blockSize=n), NAMES["r2s"], context=ctx, te=te)
             for n in (512, 128))
     assert np.array_equal(a["final_theta"], b["final_theta"])
+
+
+def _match(ctx, y, D, w=None):
+    y, D = np.ascontiguousarray(y, np.float32), np.ascontiguousarray(D, np.float32)
+    w = None if w is None else np.ascontiguousarray(w, np.float32)
+    best, sse = np.full(y.shape[1], -7, np.int32), np.full(y.shape[1], np.nan, np.float32)
+    _lib.check(_lib.lib().gx_dictionary_match(ctx.ptr, _lib.MEM_HOST, y.ctypes.data, y.shape[1], D.ctypes.data,
+                                              D.shape[1], y.shape[0], None if w is None else w.ctypes.data,
+                                              best.ctypes.data, sse.ctypes.data))
+    return best, sse
+
+
+def _scores(y, D, w=None):
+    """sse [voxel, entry] in FP64 by the expanded form; NaN for an entry without a norm."""
+    y, D = np.asarray(y, np.float32).astype(np.float64), np.asarray(D, np.float32).astype(np.float64)
+    w = np.ones((y.shape[0], 1)) if w is None else np.asarray(w, np.float32).astype(np.float64)[:, None]
+    with np.errstate(divide="ignore", invalid="ignore", over="ignore"):
+        c = (y.T @ D) / (D * D).sum(0)
+        return (w * y * y).sum(0)[:, None] - c * (2 * (w * y).T @ D - c * (w * D * D).sum(0))
+
+
+@pytest.mark.parametrize("nm", [1, 8, 9, 16, 17, 24, 33, 56, 64, 65])
+@pytest.mark.parametrize("nvox,entries", [(1, 127), (127, 128), (129, 129), (260, 1000)])
+def test_dictionary_tiles(ctx, nm, nvox, entries):
+    """Both kernels around their rule (64 measurements, 128 entries) and around
+    the 128-row operand tiles, at scales from 1e-20 to 1e20: the entry of least
+    FP64 score, or one whose score equals it to 1e-12 of the voxel's energy."""
+    rng = np.random.default_rng(nm * 1000 + nvox)
+    y = rng.standard_normal((nm, nvox)) * 10.0 ** rng.uniform(-10, 10, nvox)
+    D = rng.standard_normal((nm, entries)) * 10.0 ** rng.uniform(-10, 10, entries)
+    best, sse = _match(ctx, y, D)
+    s = _scores(y, D)
+    A = (np.asarray(y, np.float32).astype(np.float64) ** 2).sum(0)
+    got = s[np.arange(nvox), best]
+    assert np.all(got - s.min(1) <= 1e-12 * A)
+    assert np.all(np.abs(sse - got) <= 1e-6 * np.abs(got) + 1e-12 * A)
+
+
+def test_dictionary_special_values(ctx):
+    """Zero voxels take the first entry with a norm, voxels and entries that are
+    not numbers match nothing, of equal entries the first wins, and voxels with
+    too many near-identical entries for the kept list are still exact."""
+    rng = np.random.default_rng(8)
+    D = np.abs(rng.standard_normal((12, 600))) + 0.1
+    D[:, 0] = 0.0
+    D[3, 1], D[4, 2] = np.nan, np.inf
+    D[:, 300:400] = D[:, 200:300]
+    y = D[:, rng.integers(200, 600, 150)] * 3.0 + 0.01 * rng.standard_normal((12, 150))
+    y[:, 0] = 0.0
+    y[5, 1], y[6, 2] = np.nan, np.inf
+    best, sse = _match(ctx, y, D)
+    assert best[0] == 3 and sse[0] == 0.0
+    assert best[1] == best[2] == -1 and np.all(np.isinf(sse[1:3]))
+    assert np.array_equal(best[3:], np.nanargmin(_scores(y[:, 3:], D), axis=1))
+    assert not np.any((best >= 300) & (best < 400))
+    # a fine one-parameter dictionary in random order: many entries within the tensor cores' error
+    te = np.linspace(2e-3, 40e-3, 12)[:, None]
+    fine = np.exp(-te * rng.permutation(np.linspace(20.0, 20.2, 4000)))
+    y = np.exp(-te * rng.uniform(20.0, 20.2, 700)) + 1e-3 * rng.standard_normal((12, 700))
+    for n in (5, 700):
+        best, _ = _match(ctx, y[:, :n], fine)
+        s = _scores(y[:, :n], fine)
+        A = (np.asarray(y[:, :n], np.float32).astype(np.float64) ** 2).sum(0)
+        assert np.all(s[np.arange(n), best] - s.min(1) <= 1e-12 * A)
