@@ -1527,6 +1527,65 @@ extern "C" gx_status gx_askadam(gx_context* c, const gx_model* model, int32_t me
     return st;
 }
 
+// The evaluation without a regulariser: one kernel on the caller's device
+// arrays, or on contiguous device copies of host arrays; no fit state is set up.
+static gx_status gradient_direct(AdamJob& J, const float* theta, float* gtheta, float* residual, double* loss,
+                                 double* loss_fid, double* loss_reg, long long launches0) {
+    gx_context* c = J.c;
+    const gx_askadam_opts* o = J.o;
+    const gx_volume& v = J.vols[0];
+    const size_t n = v.nvox;
+    if (o->block_size > 0 && (o->block_size % 32 || o->block_size > 1024))
+        return fail(GX_EINVAL, "block_size must be a multiple of 32 in [32,1024]");
+    AdamParams a;
+    memset(&a, 0, sizeof(a));
+    a.P = make_protocol(J.model, J.id, J.np, J.nm, o->lb, o->ub, J.np);
+    make_nodes(a.P, &a.nodes);
+    a.nm = J.nm;
+    a.np = J.np;
+    a.nvtot = v.nvox;
+    a.mse_scale = (float)o->mse_scale;
+    a.huber_delta = (float)o->huber_delta;
+    a.sigma_default = (float)o->sigma;
+    const bool host = copy_kind_host(J.mem);
+    // a host array's copy on the device, or the caller's device array
+    auto in = [&](Slot s, const float* p, int rows, const float** out) -> gx_status {
+        *out = p;
+        if (!host || !p) return GX_OK;
+        float* d;
+        TRY(wsT(c, s, rows * n, &d));
+        TRY(upload_rows(c, d, n, 0, p, rows, (int)n, J.mem, &J.h2d));
+        *out = d;
+        return GX_OK;
+    };
+    const float* th;
+    TRY(in(S_DATA, v.data, J.nm, &a.data));
+    TRY(in(S_W, v.weights, J.nm, &a.weights));
+    TRY(in(S_B1, v.b1, 1, &a.b1));
+    TRY(in(S_SIG, v.sigma, 1, &a.sigma));
+    TRY(in(S_P_TH, theta, J.np, &th));
+    float *g = gtheta, *res = residual;
+    if (host && gtheta) TRY(wsT(c, S_P_GTH, (size_t)J.np * n, &g));
+    if (host && residual) TRY(wsT(c, S_P_RES, (size_t)J.nm * n, &res));
+    a.res_out = res;
+    double* total;
+    TRY(wsT(c, S_P_ACC, 8, &total));
+    double* out;
+    TRY(pinned(c, sizeof(double), (void**)&out));
+    CK(cudaMemsetAsync(total, 0, sizeof(double), c->stream));
+    const double normd = 1.0 / ((double)J.nm * (double)n);
+    CK(launch_gradient(a, J.id, o->loss, th, g, (float)normd, normd, total, c->stream));
+    CK(cudaMemcpyAsync(out, total, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    if (host && gtheta) TRY(download_rows(c, gtheta, g, n, 0, J.np, (int)n, J.mem, &J.d2h));
+    if (host && residual) TRY(download_rows(c, residual, res, n, 0, J.nm, (int)n, J.mem, &J.d2h));
+    CK(cudaStreamSynchronize(c->stream));
+    if (loss) *loss = *out;
+    if (loss_fid) *loss_fid = *out;
+    if (loss_reg) *loss_reg = 0.0;
+    c->timing.kernel_launches = g_kernel_launches - launches0;
+    return GX_OK;
+}
+
 // One evaluation of loss and d loss / d theta at physical parameters theta
 // (askadam.model_gradient, utils/askadam.m:23-117).
 extern "C" gx_status gx_model_gradient(gx_context* c, const gx_model* model, int32_t mem,
@@ -1539,6 +1598,7 @@ extern "C" gx_status gx_model_gradient(gx_context* c, const gx_model* model, int
     J.c = c; J.model = model; J.o = opts; J.mem = mem; J.vols = vol; J.nvol = 1;
     TRY(model_sizes(model, &J.np, &J.nm, &J.id));
     TRY(validate_adam(opts, J.np, vol, 1, J.nm));
+    if (!(opts->n_reg > 0 && opts->lambda[0] > 0)) return gradient_direct(J, theta, gtheta, residual, loss, loss_fid, loss_reg, scope.launches0);
     gx_askadam_opts o2 = *opts;
     o2.iteration = 0;
     J.o = &o2;

@@ -151,6 +151,10 @@ cudaError_t launch_robust_seed(const AdamParams& a, const PlainBufs& b, int wind
                                cudaStream_t s);
 cudaError_t launch_robust_check(const AdamParams& a, const PlainBufs& b, int slot, int oldest,
                                 const RobustOpts& ro, int nvox, int block, int nblocks, cudaStream_t s);
+// One gradient evaluation on the arrays of `a` with stride a.nvtot (no padding, no regulariser);
+// *total += the loss; gtheta, a.res_out may be nullptr.
+cudaError_t launch_gradient(const AdamParams& a, int model, int loss, const float* theta, float* gtheta, float norm,
+                            double normd, double* total, cudaStream_t s);
 cudaError_t launch_robust_window(const AdamParams& a, const PlainBufs& b, int block, int nblocks, cudaStream_t s);
 cudaError_t launch_robust_conv(const AdamParams& a, const PlainBufs& b, int block, int nblocks, cudaStream_t s);
 

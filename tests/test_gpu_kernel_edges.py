@@ -163,3 +163,43 @@ def test_dictionary_special_values(ctx):
         s = _scores(y[:, :n], fine)
         A = (np.asarray(y[:, :n], np.float32).astype(np.float64) ** 2).sum(0)
         assert np.all(s[np.arange(n), best] - s.min(1) <= 1e-12 * A)
+
+
+@pytest.mark.parametrize("kind", ["r2s", "r1r2s", "nexi", "nexi2"])
+@pytest.mark.parametrize("n", [1, 127, 129])
+def test_gradient_on_device_arrays(ctx, kind, n):
+    """The one-kernel gradient: device and host arrays, weights, a missing
+    gradient or residual, against the oracle (the gradient parity test's bars)."""
+    import torch
+    rng = np.random.default_rng(n)
+    gxm, om = models(kind)
+    lb, ub = bounds(kind)
+    th = random_theta(kind, n, rng).astype(np.float32)
+    s = oracle.forward(om, th.astype(np.float64))
+    y = (s + 0.02 * rng.standard_normal(s.shape)).astype(np.float32)
+    w = rng.uniform(0.2, 1.0, y.shape).astype(np.float32)
+    f = fitting(lossFunction="l2")
+    opts = gx_askadam.build_opts(f, NAMES[kind], lb, ub)
+    Lo, go, ro, _, _ = oracle.model_gradient(om, oracle.Volume(y.astype(np.float64), weights=w.astype(np.float64)),
+                                             oracle.adam_opts(lb, ub, f), th.astype(np.float64))
+    fp = lambda t: C.cast(C.c_void_p(t.data_ptr()), _lib._fp)  # noqa: E731
+    arrays = {}
+    for mem in (_lib.MEM_HOST, _lib.MEM_DEVICE):
+        dev = "cuda" if mem == _lib.MEM_DEVICE else "cpu"
+        ty, tw, tt = (torch.from_numpy(x).to(dev).contiguous() for x in (y, w, th))
+        g, r, loss = torch.full_like(tt, -7.0), torch.full_like(ty, -7.0), C.c_double()
+        vol = _lib.GxVolume()
+        vol.dims[0], vol.dims[1], vol.dims[2], vol.nvox = n, 1, 1, n
+        vol.data, vol.weights = fp(ty), fp(tw)
+        torch.cuda.synchronize()
+        for gp, rp in ((g.data_ptr(), r.data_ptr()), (None, r.data_ptr()), (g.data_ptr(), None)):
+            _lib.check(_lib.lib().gx_model_gradient(ctx.ptr, C.byref(gxm.s), mem, C.byref(vol), C.byref(opts),
+                                                    tt.data_ptr(), gp, rp, C.byref(loss), None, None))
+        arrays[mem] = (g.cpu().numpy(), r.cpu().numpy(), loss.value)
+    for a, b in zip(*arrays.values()):
+        assert np.allclose(a, b, rtol=1e-12, atol=0.0)
+    g, r, loss = arrays[_lib.MEM_HOST]
+    assert abs(loss - Lo) <= 1e-5 * abs(Lo) + 1e-7
+    assert np.all(np.abs(r - ro) <= 2e-4 * np.abs(ro) + 2e-5)
+    for k in range(th.shape[0]):
+        assert np.max(np.abs(g[k] - go[k])) <= 1e-3 * np.max(np.abs(go[k])) + 1e-12
