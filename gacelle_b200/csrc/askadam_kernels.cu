@@ -1061,6 +1061,9 @@ int fused_block_limit(const AdamParams& a, int model, int loss, bool stats) {
 cudaError_t launch_fused(const AdamParams& a, int model, int loss, bool stats, int e_begin,
                          int e_end, int update_last, bool record, int block, int nblocks,
                          cudaStream_t s) {
+    const FusedKind kind = fused_kind(a, model, loss, block);
+    if (kind != kFusedGeneral)
+        return launch_fused_std(kind, a, stats, e_begin, e_end, update_last, record, block, nblocks, s);
 #define GX_F(M)                                                                                    \
     return stats ? fused_dispatch2<M, true>(a, loss, e_begin, e_end, update_last, record, block, nblocks, s) \
                  : fused_dispatch2<M, false>(a, loss, e_begin, e_end, update_last, record, block, nblocks, s)

@@ -572,6 +572,14 @@ __device__ __forceinline__ void r1r2s_mse_sums(const DevProtocol& P, float R2, i
     }
 }
 
+// The steady-state factor A = sin a (1 - E1) / (1 - cos a E1) of one flip angle
+// and dA/dR1 (sa, ca: sine and cosine of the voxel's angle).
+__device__ __forceinline__ void r1r2s_angle(float sa, float ca, float tr, float E1, float& A, float& dA) {
+    const float inv = 1.0f / (1.0f - ca * E1);
+    A = sa * (1.0f - E1) * inv;
+    dA = sa * (ca - 1.0f) * inv * inv * (-tr * E1);
+}
+
 template <int NFA, bool EXACT, int NTE, class Acc>
 __device__ __forceinline__ void r1r2s_mse(const DevProtocol& P, float M0, float R1, float R2, const VoxAux& va,
                                           Acc& acc) {
@@ -582,10 +590,7 @@ __device__ __forceinline__ void r1r2s_mse(const DevProtocol& P, float M0, float 
     for (int f = 0; f < NFA; ++f) {
         A[f] = dA[f] = AM0[f] = 0.0f;
         if (EXACT || f < nfa) {
-            const float sa = va.sa[f * va.fs], ca = va.ca[f * va.fs];
-            const float inv = 1.0f / (1.0f - ca * E1);
-            A[f] = sa * (1.0f - E1) * inv;
-            dA[f] = sa * (ca - 1.0f) * inv * inv * (-P.tr * E1);
+            r1r2s_angle(va.sa[f * va.fs], va.ca[f * va.fs], P.tr, E1, A[f], dA[f]);
             AM0[f] = mul1(A[f], M0);
         }
         Sq[f] = 0.0f;
@@ -1058,6 +1063,13 @@ struct PairConsts {
     float2 mse, s2;   // mse_scale, 2 mse_scale
     float2 iv[3];     // inverse voxel sizes
     float2 niv[3];    // their negatives
+};
+
+// The same for the kernels of fits without spatial coupling (up to three parameters).
+struct FusedPairConsts {
+    float2 nl2e, one, rng[3], lb[3];
+    float2 b1, omb1, b2, omb2, eps;
+    float2 mse, s2;
 };
 
 // The sigmoid transform of a pair of voxels with its constants from

@@ -151,6 +151,12 @@ cudaError_t launch_robust_seed(const AdamParams& a, const PlainBufs& b, int wind
                                cudaStream_t s);
 cudaError_t launch_robust_check(const AdamParams& a, const PlainBufs& b, int slot, int oldest,
                                 const RobustOpts& ro, int nvox, int block, int nblocks, cudaStream_t s);
+// The kernels of askadam_fused.cu and the rule between them and the general one.
+enum FusedKind { kFusedGeneral, kFusedR2s, kFusedR2sPairs, kFusedR1r2sPairs };
+constexpr int kPairVoxels = 148 * 512;
+FusedKind fused_kind(const AdamParams& a, int model, int loss, int block);
+cudaError_t launch_fused_std(FusedKind kind, const AdamParams& a, bool stats, int e_begin, int e_end, int update_last,
+                             bool record, int block, int nblocks, cudaStream_t s);
 // One gradient evaluation on the arrays of `a` with stride a.nvtot (no padding, no regulariser);
 // *total += the loss; gtheta, a.res_out may be nullptr.
 cudaError_t launch_gradient(const AdamParams& a, int model, int loss, const float* theta, float* gtheta, float norm,

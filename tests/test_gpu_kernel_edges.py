@@ -165,6 +165,57 @@ def test_dictionary_special_values(ctx):
         assert np.all(s[np.arange(n), best] - s.min(1) <= 1e-12 * A)
 
 
+def _std_fit(ctx, kind, n, te, block, iters, **over):
+    from helpers import run_engine
+    rng = np.random.default_rng(n)
+    _, om = models(kind, te=te)
+    y = oracle.forward(om, random_theta(kind, n, rng)) + 0.01 * rng.standard_normal((len(te) * (1 + (kind != "r2s")), n))
+    th0 = np.tile(np.array([[1.0], [30.0]] if kind == "r2s" else [[1.0], [1.0], [30.0]], np.float32), (1, n))
+    return run_engine(kind, y, th0, fitting(iteration=iters, blockSize=block, **over), NAMES[kind], context=ctx, te=te)
+
+
+def _same_fit(a, b, iters):
+    for k in ("final_theta", "min_theta", "final_residual", "min_residual"):
+        assert np.array_equal(a[k], b[k]), k
+    assert a["final_niteration"] == b["final_niteration"] and a["min_niteration"] == b["min_niteration"]
+    # the history's per-voxel terms are equal, their FP32 sums over a warp in another order (32 terms: 32 x 2^-24)
+    h, g = a["loss_history"][: iters + 1], b["loss_history"][: iters + 1]
+    assert np.allclose(h, g, rtol=4e-6, atol=0.0, equal_nan=True)
+
+
+@pytest.mark.parametrize("n_te", [1, 8, 9, 12, 13, 16, 17])
+@pytest.mark.parametrize("kind", ["r2s", "r1r2s"])
+def test_fused_kernels_equal_the_general_one(ctx, kind, n_te):
+    """The kernels of the standard configuration give the general kernel's
+    parameters bit for bit: below, at and above their echo bounds, with volumes
+    that end inside a 64-voxel chunk (the general kernel takes 96-thread blocks of R1-R2* and
+    1024-thread blocks of R2*)."""
+    te = np.linspace(2e-3, 40e-3, n_te) if n_te > 1 else np.array([5e-3])
+    general = 1024 if kind == "r2s" else 96
+    for n in (1, 33, 450):
+        _same_fit(_std_fit(ctx, kind, n, te, 64, 40), _std_fit(ctx, kind, n, te, general, 40), 40)
+
+
+@pytest.mark.parametrize("iters", [0, 1, 2, 31, 32, 33, 65])
+@pytest.mark.parametrize("block", [32, 64, 128, 512])
+def test_history_groups(ctx, iters, block):
+    """Loss history and stopping statistics of fits that end around a group of
+    32 epochs, with one and several warps a block (several volumes' worth of blocks)."""
+    te = np.linspace(2e-3, 40e-3, 12)
+    over = {"convergenceStepTol": 1e-30, "convergenceGradTol": 1e-30}
+    for kind, general in (("r2s", 1024), ("r1r2s", 96)):
+        a = _std_fit(ctx, kind, 700, te, block, iters, **over)
+        _same_fit(a, _std_fit(ctx, kind, 700, te, general, iters, **over), iters)
+        assert np.all(np.isfinite(a["loss_history"]))
+
+
+@pytest.mark.parametrize("n", [75_700, 75_800])
+def test_r2s_pairs_rule(ctx, n):
+    """Around the voxel count from which R2* takes two voxels a thread."""
+    te = np.linspace(2e-3, 40e-3, 12)
+    _same_fit(_std_fit(ctx, "r2s", n, te, 128, 33), _std_fit(ctx, "r2s", n, te, 1024, 33), 33)
+
+
 @pytest.mark.parametrize("kind", ["r2s", "r1r2s", "nexi", "nexi2"])
 @pytest.mark.parametrize("n", [1, 127, 129])
 def test_gradient_on_device_arrays(ctx, kind, n):
