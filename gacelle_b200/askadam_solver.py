@@ -215,8 +215,9 @@ class askadam:
     check_set_default_basic = staticmethod(check_set_default_basic)
 
     def optimisation(self, data, mask, weights, parameters, fitting, userfuncCell, *varargin,
-                     extradata=None):
-        """askadam.optimisation (utils/askadam.m:121-365)."""
+                     extradata=None, masked=None):
+        """askadam.optimisation (utils/askadam.m:121-365).  masked: the data's
+        masked [Nmeas, Nvox] matrix (utils.to_GD), where the caller has it."""
         model = _model_of(userfuncCell)
         fitting = check_set_default_basic(fitting)
         prior = surface = None
@@ -238,7 +239,7 @@ class askadam:
         mask = np.asarray(mask)
         d3 = utils.dims3(mask)
         idx = utils.mask_index(mask)
-        y = utils.to_GD(data, mask, idx).astype(np.float32)
+        y = (utils.to_GD(data, mask, idx) if masked is None else masked).astype(np.float32, copy=False)
         nm, nv = y.shape
         model_params = list(fitting.get("modelParams") or model.modelParams)
         np_ = len(model_params)
@@ -269,7 +270,7 @@ class askadam:
         pr = self._prior_maps(prior, fitting, mask, idx, nv) if prior is not None and opts.n_reg > 0 else None
         sf = self._surface_tables(surface, mask, idx) if surface is not None and opts.n_reg > 0 else None
         res = self._run(gxm, y, w, theta0, b1, sig, gidx, d3, opts, nm, np_, pr, sf)
-        return self._to_out(res, model_params, mask, fitting, nm, nv)
+        return self._to_out(res, model_params, mask, fitting, nm, nv, idx)
 
     @staticmethod
     def _prior_maps(prior, fitting, mask, idx, nv):
@@ -370,19 +371,20 @@ class askadam:
         return out
 
     @staticmethod
-    def _to_out(res, model_params, mask, fitting, nm, nv):
+    def _to_out(res, model_params, mask, fitting, nm, nv, idx=None):
         """Output structure of utils/askadam.m:327-362."""
         out = {"final": {}, "min": {}}
         shape = np.shape(mask)
+        idx = utils.mask_index(mask) if idx is None else idx
         for k, p in enumerate(model_params):
             for which in ("final", "min"):
-                out[which][p] = utils.reshape_GD2ND(res[f"{which}_theta"][k], mask).reshape(shape, order="F")
+                out[which][p] = utils.reshape_GD2ND(res[f"{which}_theta"][k], mask, idx).reshape(shape, order="F")
         for which in ("final", "min"):
             o = out[which]
             o["loss"] = res[f"{which}_loss"]
             o["loss_fidelity"] = res[f"{which}_loss_fidelity"]
             o["loss_reg"] = res[f"{which}_loss_reg"]
-            o["resloss"] = utils.reshape_GD2ND(res[f"{which}_resloss"], mask).reshape(shape, order="F")
+            o["resloss"] = utils.reshape_GD2ND(res[f"{which}_resloss"], mask, idx).reshape(shape, order="F")
             o["residual"] = res[f"{which}_residual"]
             o["Niteration"] = res[f"{which}_niteration"]
         out["final"]["memoryUsage"] = 0.0

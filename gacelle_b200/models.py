@@ -143,12 +143,13 @@ class _ModelBase:
             return s
         return s.T.reshape(shape + (s.shape[0],), order="F")
 
-    def _solve(self, data, mask, w, pars0, fitting, extradata=None):
+    def _solve(self, data, mask, w, pars0, fitting, extradata=None, masked=None):
+        """masked: the data's masked [Nmeas, Nvox] matrix, where the caller has it."""
         from .askadam_solver import askadam
         from .mcmc_solver import mcmc
         if fitting["solver"] == "askadam":
             return askadam(self.context, fitting.get("path", "fused")).optimisation(
-                data, mask, w, pars0, fitting, self, extradata=extradata)
+                data, mask, w, pars0, fitting, self, extradata=extradata, masked=masked)
         fitting = dict(fitting)
         fitting["xStepSize"] = list(self.step)
         return mcmc(self.context).optimisation(data, mask, w, pars0, fitting, self, extradata=extradata)
@@ -260,10 +261,30 @@ class gpuR2starMapping(_ModelBase):
             fitting["ub"] = self.ub[: len(self.modelParams)]
         if not len(fitting["lb"]):
             fitting["lb"] = self.lb[: len(self.modelParams)]
-        pars0 = self.determine_x0(data, mask, fitting)
-        w = self.compute_optimisation_weights(data, fitting)
-        w = None if np.all(w == 1) else w
-        return self._solve(data, mask, w, pars0, fitting)
+        masked = None
+        if str(fitting["start"]).lower() == "prior" and data.ndim == 4 and tuple(data.shape[:3]) == utils.dims3(mask):
+            masked = utils.to_GD(data, mask)
+            pars0 = self._masked_prior(masked, fitting)
+        else:
+            pars0 = self.determine_x0(data, mask, fitting)
+        w = None
+        if fitting["isWeighted"]:
+            w = self.compute_optimisation_weights(data, fitting)
+            w = None if np.all(w == 1) else w
+        return self._solve(data, mask, w, pars0, fitting, masked=masked)
+
+    def _masked_prior(self, y, fitting):
+        """determine_x0's prior start for the voxels of the mask alone (y: [Nmeas,
+        Nvox]), as [1, Nvox] rows: estimate_prior's operations voxel by voxel,
+        without the image outside the mask, in stretches whose echoes stay in
+        the cache."""
+        r2 = np.empty(y.shape[1])
+        for i in range(0, y.shape[1], 8192):
+            r2[i:i + 8192] = self.R2star_trapezoidal(y[:, i:i + 8192].T, self.te)
+        bad = ~np.isfinite(r2) | (r2 < self.lb[1])
+        r2 = np.where(bad, self.lb[1], np.minimum(r2, self.ub[1]))
+        x0 = {"M0": np.abs(y[:1]).astype(np.float32), "R2star": r2[None].astype(np.float32)}
+        return {p: np.clip(v, fitting["lb"][k], fitting["ub"][k]) for k, (p, v) in enumerate(x0.items())}
 
     def estimate(self, data, mask, fitting=None):
         """R2star/gpuR2starMapping.m:94-179: scaled data, fit (in

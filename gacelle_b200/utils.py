@@ -20,7 +20,8 @@ def dims3(mask) -> tuple:
 
 def mask_index(mask) -> np.ndarray:
     """find(mask > 0) as 0-based column-major linear indices."""
-    return np.flatnonzero(np.asarray(mask).ravel(order="F") > 0).astype(np.int64)
+    m = np.asarray(mask).ravel(order="F")
+    return np.flatnonzero(m if m.dtype == bool else m > 0).astype(np.int64, copy=False)
 
 
 def reshape_ND2GD(data, mask_idx) -> np.ndarray:
@@ -28,7 +29,7 @@ def reshape_ND2GD(data, mask_idx) -> np.ndarray:
     data = np.asarray(data)
     d3 = dims3(data)
     flat = data.reshape((d3[0] * d3[1] * d3[2], -1), order="F")
-    return np.ascontiguousarray(flat[mask_idx].T)
+    return np.take(flat.T, mask_idx, axis=1)  # row by row: contiguous reads and writes
 
 
 def to_GD(data, mask, mask_idx=None) -> np.ndarray:
@@ -42,18 +43,22 @@ def to_GD(data, mask, mask_idx=None) -> np.ndarray:
     return np.ascontiguousarray(data[:, mask_idx])
 
 
-def reshape_GD2ND(gd, mask) -> np.ndarray:
+def reshape_GD2ND(gd, mask, mask_idx=None) -> np.ndarray:
     """utils.reshape_ND2image (utils/utils.m:299-315): [K, Nvox] -> image
-    [x,y,z,K] with zeros outside the mask ([x,y,z] when K == 1)."""
+    [x,y,z,K] with zeros outside the mask ([x,y,z] when K == 1).  mask_idx:
+    mask_index(mask), where the caller has it."""
     gd = np.asarray(gd)
     if gd.ndim == 1:
         gd = gd[None, :]
     d3 = dims3(mask)
-    idx = mask_index(mask)
+    idx = mask_index(mask) if mask_idx is None else mask_idx
+    if gd.shape[0] == 1:
+        img = np.zeros(d3[0] * d3[1] * d3[2], dtype=gd.dtype)
+        img[idx] = gd[0]
+        return img.reshape(d3, order="F")
     img = np.zeros((d3[0] * d3[1] * d3[2], gd.shape[0]), dtype=gd.dtype)
     img[idx] = gd.T
-    img = img.reshape(d3 + (gd.shape[0],), order="F")
-    return img[..., 0] if gd.shape[0] == 1 else img
+    return img.reshape(d3 + (gd.shape[0],), order="F")
 
 
 def param_to_GD(value, mask, mask_idx, nvox) -> np.ndarray:
