@@ -19,9 +19,11 @@
 // another: a worker warp arrives on a shared-memory mbarrier (with its
 // partial loss-history sums) after its map writes, runs its next fidelity
 // pass, and waits only before its next TV/update pass.  The CTA's last warp
-// is a barrier warp: it collects the worker arrivals, adds the epoch's loss
-// history, runs the grid barrier and opens the next TV/update pass (a second
-// mbarrier).  Every wait is bounded: if one expires the kernel raises an
+// is a barrier warp: it collects the worker arrivals, runs the grid barrier,
+// opens the next TV/update pass (a second mbarrier) and then adds the epoch's
+// loss history, which nobody waits for (opening after the history, and a butterfly
+// for each of its quantities in the workers, took 27.5 ms for 4000 epochs of 629,432
+// voxels and 3.1 us an epoch of a small volume; now 26.7 ms and 2.9 us).  Every wait is bounded: if one expires the kernel raises an
 // error flag that the host reports as GX_ETIMEOUT, and every CTA returns.
 //
 // The per-voxel arithmetic (forward model, loss, adjoint, TV subgradient,
@@ -218,33 +220,41 @@ struct HaloMap {
 // a time.
 // Threads per CTA at most: the 32-echo variant and the pair variants (two
 // voxels' measurements per thread) need more than 64 registers.
-__host__ __device__ constexpr bool persist_pairs(int maxm, bool stats) { return maxm > 0 && maxm <= 16 && !stats; }
-__host__ __device__ constexpr int persist_max_threads(int maxm, bool stats) {
-    return (maxm > 16 || persist_pairs(maxm, stats)) ? 768 : kPersistMaxThreads;
+__host__ __device__ constexpr bool persist_can_pair(int maxm) { return maxm > 0 && maxm <= 16; }
+// Two voxels per thread: without statistics always; with them from slices of
+// kPairStatsSlice voxels on.  200 epochs, one voxel a thread / pairs: slices of 65
+// voxels 0.63 / 0.65 ms, 292: 0.68 / 0.70, 532: 0.77 / 0.74, 1168: 1.01 /
+// 0.84, 4251: 2.46 / 1.62 (small slices gain more from the larger number of
+// warps).
+constexpr int kPairStatsSlice = 448;
+inline bool persist_pairs(int maxm, bool stats, int slice) {
+    return persist_can_pair(maxm) && (!stats || slice >= kPairStatsSlice);
 }
+__host__ __device__ constexpr int persist_max_threads(int maxm) { return maxm > 0 ? 768 : kPersistMaxThreads; }
 
 // HOOK: the bound of the waits and the grid barrier's arrival count come from
 // the launch arguments (the context's test hooks); otherwise they are the
 // compile-time default, which keeps the wait loops of the timed kernel lean.
-template <int LOSS, bool STATS, int MAXM, bool HOOK>
-__global__ void __launch_bounds__(persist_max_threads(MAXM, STATS), 1)
+template <int LOSS, bool STATS, int MAXM, bool PAIR, bool HOOK>
+__global__ void __launch_bounds__(persist_max_threads(MAXM), 1)
 tv_persistent_kernel(AdamParams a, PersistArgs p) {
     const long long wait_limit = HOOK ? p.spin_cycles : kBarrierSpinCycles;
     const unsigned int extra_arrivals = HOOK ? p.extra_arrivals : 0u;
     constexpr int NP = 2;  // R2*: M0, R2star
-    constexpr int NS = STATS ? 4 : 3;  // z, m1, m2 [, z of the previous epoch]
+    // z, m1, m2 [, z of the previous epoch: the pair variant adds up an
+    // update's steps as it makes them, for the next epoch's history]
+    constexpr int NS = STATS && !PAIR ? 4 : 3;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* s_red = reinterpret_cast<double*>(smem_raw);                     // [2][32][kHistW]
     float* s_st = reinterpret_cast<float*>(s_red + 2 * 32 * kHistW);         // [NS][NP][slice]
-    // CACHE: the standard configuration without statistics keeps, from the
+    // CACHE: the standard configuration up to 16 measurements keeps, from the
     // fidelity pass, the unregularised parameter's z-gradient and the
-    // regularised one's fidelity gradient (in the space the previous-epoch z
-    // takes when statistics are on), and from the update pass the regularised
-    // parameter's theta and dtheta/dz, so that no pass evaluates a transform
-    // another pass has evaluated; same operations, same order.
-    // PAIR (up to 16 measurements, without statistics): two voxels per
-    // thread, pair instructions, with the fidelity-pass cache (CACHE)
-    constexpr bool PAIR = persist_pairs(MAXM, STATS);
+    // regularised one's fidelity gradient, and from the update pass the
+    // regularised parameter's theta and dtheta/dz, so that no pass evaluates a
+    // transform another pass has evaluated; same operations, same order.
+    // PAIR (the same configuration): two voxels per thread, pair
+    // instructions, with the fidelity-pass cache (CACHE)
+    static_assert(!PAIR || persist_can_pair(MAXM), "the pair variant's measurements are in registers");
     constexpr bool CACHE = PAIR;
     constexpr int NAUX = CACHE ? 4 : NP;
     float* s_gf = s_st + (size_t)NS * NP * p.slice;                          // [NAUX][slice] fidelity pass results
@@ -324,7 +334,7 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
             s_st[(0 * NP + k) * S + j] = a.z[gi];
             s_st[(1 * NP + k) * S + j] = a.m1[gi];
             s_st[(2 * NP + k) * S + j] = a.m2[gi];
-            if constexpr (STATS) s_st[(3 * NP + k) * S + j] = a.zprev ? a.zprev[gi] : 0.0f;
+            if constexpr (NS > 3) s_st[(3 * NP + k) * S + j] = a.zprev ? a.zprev[gi] : 0.0f;
         }
         if (p.data_in_smem)
             for (int m = 0; m < a.nm; ++m) s_y[m * S + j] = a.data[(size_t)m * a.nvtot + base + i];
@@ -372,14 +382,19 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
                 }
                 return;
             }
-            // lane 31 publishes the CTA's maps and waits for the other CTAs
-            // while lanes 0-4 add the epoch's loss history
+            // the grid barrier and the opening first: the workers wait for it.
+            // The history follows; its buffer of epoch e is written again for epoch e + 2, behind the opening of
+            // e + 1, which this warp signals after it has read it
             int ok = 1;
-            if (e < p.e_end && lane == 31) {
-                grid_arrive_one(p.barrier);
-                ok = grid_wait_one(p.barrier, (unsigned int)(e - p.e_begin + 2) * gridDim.x + extra_arrivals,
-                                   wait_limit);
-                if (!ok) *(volatile int*)&s_err = 1;
+            if (e < p.e_end) {
+                if (lane == 31) {
+                    grid_arrive_one(p.barrier);
+                    ok = grid_wait_one(p.barrier, (unsigned int)(e - p.e_begin + 2) * gridDim.x + extra_arrivals,
+                                       wait_limit);
+                    if (!ok) *(volatile int*)&s_err = 1;
+                    mbar_arrive(&bar_open);
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 31);
             }
             if (p.record && a.hist && lane < NQ) {
                 const double* buf = s_red + (e & 1) * 32 * kHistW;
@@ -388,14 +403,11 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
                 if (lane == 0) t *= V.normd;
                 if (t != 0.0) atomicAdd(a.hist + ((size_t)vol * (a.niter + 1) + e) * kHistW + lane, t);
             }
-            __syncwarp();  // the history buffer of epoch e is read before epoch e+1 opens
-            if (e < p.e_end) {
-                if (lane == 31) mbar_arrive(&bar_open);
-                ok = __shfl_sync(0xffffffffu, ok, 31);
-                if (!ok) return;
-            }
+            __syncwarp();
+            if (!ok) return;
         }
-    } else
+    } else {
+    float step2 = 0.0f;  // PAIR and STATS: squared steps of the last update, this thread's voxels
     for (int e = p.e_begin; e <= p.e_end; ++e) {
         const float* gcur = (e >= 1 && ((e - 1) & 1)) ? p.grid1 : p.grid0;  // epoch 0 reads the start map
         float* gnext = e & 1 ? p.grid1 : p.grid0;
@@ -495,6 +507,11 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
         const float* G = gcur + V.hgrid_off;
         float* Gn = gnext + V.hgrid_off;
         const float2 nscx = bcast2(-sc.x), scy = bcast2(sc.y);
+        // the step that led to the evaluated state: of the previous epoch's
+        // update, or (first epoch of the launch) from the stored previous state
+        if constexpr (STATS) q4 = step2;
+        float nstep2 = 0.0f;
+        const bool last_upd = STATS && e == min(p.e_end, p.update_last);
         // pass 2: TV subgradient, chain rule, optimiser, new map values
         for (int q = tid; q < npair; q += NWT) {
             const int i0 = ((q >> 5) << 6) + (q & 31), v0 = base + i0;
@@ -521,6 +538,21 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
                 q1 = __fmaf_rn(tvs0, cost.y, q1);
                 grf.y = fma1(tvs0, gt.y, grf.y);
             }
+            if constexpr (STATS) {
+                const float2 gzr = mul2(grf, dthr);
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                    const float2 gk = k == kr ? gzr : gn, zk = ld2(s_st + k * S, q);
+                    if (ok0) { q2 = __fmaf_rn(gk.x, gk.x, q2); q3 = __fmaf_rn(zk.x, zk.x, q3); }
+                    if (ok1) { q2 = __fmaf_rn(gk.y, gk.y, q2); q3 = __fmaf_rn(zk.y, zk.y, q3); }
+                    if (e == p.e_begin && a.zprev) {
+                        const float* zp = a.zprev + (size_t)k * a.nvtot + v0;
+                        const float d0 = zk.x - zp[0], d1 = zk.y - zp[32];
+                        if (ok0) q4 = __fmaf_rn(d0, d0, q4);
+                        if (ok1) q4 = __fmaf_rn(d1, d1, q4);
+                    }
+                }
+            }
             if (upd) {
                 const float2 gzr = mul2(grf, dthr);
                 const float2 gz[NP] = {kr == 0 ? gzr : gn, kr == 0 ? gn : gzr};
@@ -531,7 +563,18 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
                     float* p1s = s_st + (1 * NP + k) * S;
                     float* p2s = s_st + (2 * NP + k) * S;
                     float2 zz = ld2(pz, q), mm1 = ld2(p1s, q), mm2 = ld2(p2s, q);
+                    const float2 zo = zz;
                     adam_step2c(p.k, nscx, scy, zz, mm1, mm2, gz[k]);
+                    if constexpr (STATS) {
+                        const float d0 = zz.x - zo.x, d1 = zz.y - zo.y;
+                        if (ok0) nstep2 = __fmaf_rn(d0, d0, nstep2);
+                        if (ok1) nstep2 = __fmaf_rn(d1, d1, nstep2);
+                        if (last_upd && a.zprev) {  // the state before the launch's last update
+                            float* zp = a.zprev + (size_t)k * a.nvtot;
+                            if (ok0) zp[v0] = zo.x;
+                            if (ok1) zp[v0 + 32] = zo.y;
+                        }
+                    }
                     st2(pz, q, zz);
                     st2(p1s, q, mm1);
                     st2(p2s, q, mm2);
@@ -557,6 +600,7 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
                 }
             }
         }
+        if constexpr (STATS) step2 = nstep2;
         return true;
         };
         bool go;
@@ -708,16 +752,30 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
         const int lane = tid & 31, warp = tid >> 5;
         if (p.record && a.hist) {
             double* buf = s_red + (e & 1) * 32 * kHistW;
-            float q[kHistW] = {q0, q1, q2, q3, q4};
-            constexpr int NQ = STATS ? kHistW : 2;
+            // butterflies at distances 16, 8, 4, 2, 1, several quantities at a
+            // time: the first exchanges leave each on its part of the lanes
+            // (the same pairs are added as with a butterfly of its own each)
+            auto merge = [&](float a0, float a1, int d) {
+                const bool second = (lane & d) != 0;
+                return (second ? a1 : a0) + __shfl_xor_sync(0xffffffffu, second ? a0 : a1, d);
+            };
+            if constexpr (STATS) {
+                float r = merge(merge(q0, q2, 16), merge(q1, q3, 16), 8);
 #pragma unroll
-            for (int k = 0; k < NQ; ++k) {
-                float sum = warp_sum_p(q[k]);
-                if (lane == 0) buf[warp * kHistW + k] = (double)sum;
+                for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+                const float s4 = warp_sum_p(q4);
+                if ((lane & 7) == 0) buf[warp * kHistW + (lane >> 4) * 2 + ((lane >> 3) & 1)] = (double)r;
+                if (lane == 0) buf[warp * kHistW + 4] = (double)s4;
+            } else {
+                float r = merge(q0, q1, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+                if ((lane & 15) == 0) buf[warp * kHistW + (lane >> 4)] = (double)r;
             }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_arrive);
+    }
     }
     __syncthreads();
     if constexpr (STD) {
@@ -760,7 +818,7 @@ tv_persistent_kernel(AdamParams a, PersistArgs p) {
             a.z[gi] = s_st[(0 * NP + k) * S + j];
             a.m1[gi] = s_st[(1 * NP + k) * S + j];
             a.m2[gi] = s_st[(2 * NP + k) * S + j];
-            if constexpr (STATS)
+            if constexpr (NS > 3)
                 if (a.zprev) a.zprev[gi] = s_st[(3 * NP + k) * S + j];
         }
     }
@@ -784,11 +842,13 @@ int persist_variant(const AdamParams& a, int loss, bool res_after_loop) {
 }
 
 template <int LOSS, int MAXM>
-cudaError_t launch_persist_t(const AdamParams& a, PersistArgs p, int bt, int nblocks, size_t smem,
+cudaError_t launch_persist_t(const AdamParams& a, PersistArgs p, bool pairs, int bt, int nblocks, size_t smem,
                              cudaStream_t s) {
     const bool hook = p.spin_cycles != kBarrierSpinCycles || p.extra_arrivals != 0;
-    auto k = p.stats ? (hook ? tv_persistent_kernel<LOSS, true, MAXM, true> : tv_persistent_kernel<LOSS, true, MAXM, false>)
-                     : (hook ? tv_persistent_kernel<LOSS, false, MAXM, true> : tv_persistent_kernel<LOSS, false, MAXM, false>);
+    constexpr bool CAN = persist_can_pair(MAXM);  // the pairs are the only variant without statistics
+    auto k = hook ? tv_persistent_kernel<LOSS, false, MAXM, CAN, true> : tv_persistent_kernel<LOSS, false, MAXM, CAN, false>;
+    if (p.stats && pairs) k = hook ? tv_persistent_kernel<LOSS, true, MAXM, CAN, true> : tv_persistent_kernel<LOSS, true, MAXM, CAN, false>;
+    else if (p.stats) k = hook ? tv_persistent_kernel<LOSS, true, MAXM, false, true> : tv_persistent_kernel<LOSS, true, MAXM, false, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<void*>(static_cast<const void*>(&a)), static_cast<void*>(&p)};
@@ -800,14 +860,19 @@ cudaError_t launch_persist_t(const AdamParams& a, PersistArgs p, int bt, int nbl
 template <int LOSS, int MAXM>
 int occupancy_t(int bt, size_t smem) {
     int nb = 0, nb2 = 0;
-    auto k0 = tv_persistent_kernel<LOSS, false, MAXM, false>;
-    auto k1 = tv_persistent_kernel<LOSS, true, MAXM, false>;
+    constexpr bool CAN = persist_can_pair(MAXM);
+    auto k0 = tv_persistent_kernel<LOSS, false, MAXM, CAN, false>;
+    auto k1 = tv_persistent_kernel<LOSS, true, MAXM, false, false>;
+    auto k2 = tv_persistent_kernel<LOSS, true, MAXM, CAN, false>;
+    int nb3 = 0;
     if (cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k0, bt, smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, k1, bt, smem) != cudaSuccess) return 0;
-    return nb < nb2 ? nb : nb2;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb3, k2, bt, smem) != cudaSuccess) return 0;
+    return std::min(nb, std::min(nb2, nb3));
 }
 
 int occupancy_v(int variant, int bt, size_t smem) {
@@ -860,10 +925,9 @@ bool plan_persistent(const AdamParams& a, int model, int loss, bool stats, int p
     // the last pass over the slice is full (every worker warp reaches the
     // grid barrier after the same number of voxels)
     const int variant = persist_variant(a, loss, true);
-    const bool pairs = persist_pairs(variant, stats) && pair_layout_ok(a.nvtot, slice);  // two voxels per thread
+    const bool pairs = persist_pairs(variant, stats, slice) && pair_layout_ok(a.nvtot, slice);  // two voxels per thread
     const int units = pairs ? slice / 2 : slice;
-    // every variant that may run with this thread count must allow it
-    const int maxw = std::min(persist_max_threads(variant, stats), persist_max_threads(variant, !stats)) - 32;
+    const int maxw = persist_max_threads(variant) - 32;
     int passes = (units + maxw - 1) / maxw;
     int bt = ((units + passes - 1) / passes + 31) / 32 * 32 + 32;
     int nb = occupancy_v(variant, bt, smem);
@@ -909,14 +973,14 @@ cudaError_t launch_tv_persistent(const AdamParams& a, const PersistPlan& plan, P
     // the pair variant needs slices and a work-list of whole 64-voxel chunks;
     // otherwise the run-time variant takes the launch
     int var = variant;
-    if (persist_pairs(var, p.stats != 0) && !pair_layout_ok(a.nvtot, plan.slice)) var = 0;
-    const int pairs = persist_pairs(var, p.stats != 0) ? 1 : 0;
+    if (persist_pairs(var, p.stats != 0, plan.slice) && !pair_layout_ok(a.nvtot, plan.slice)) var = 0;
+    const int pairs = persist_pairs(var, p.stats != 0, plan.slice) ? 1 : 0;
     if (var != plan.quad_width || pairs != plan.quad_pairs) p.data_quads = nullptr;  // read [nm][nvtot]
-    if (var == 8) return launch_persist_t<kMSE, 8>(a, p, plan.threads, plan.ctas, plan.smem, s);
-    if (var == 12) return launch_persist_t<kMSE, 12>(a, p, plan.threads, plan.ctas, plan.smem, s);
-    if (var == 16) return launch_persist_t<kMSE, 16>(a, p, plan.threads, plan.ctas, plan.smem, s);
-    if (var == 32) return launch_persist_t<kMSE, 32>(a, p, plan.threads, plan.ctas, plan.smem, s);
-    return launch_persist_t<-1, 0>(a, p, plan.threads, plan.ctas, plan.smem, s);
+    if (var == 8) return launch_persist_t<kMSE, 8>(a, p, pairs != 0, plan.threads, plan.ctas, plan.smem, s);
+    if (var == 12) return launch_persist_t<kMSE, 12>(a, p, pairs != 0, plan.threads, plan.ctas, plan.smem, s);
+    if (var == 16) return launch_persist_t<kMSE, 16>(a, p, pairs != 0, plan.threads, plan.ctas, plan.smem, s);
+    if (var == 32) return launch_persist_t<kMSE, 32>(a, p, pairs != 0, plan.threads, plan.ctas, plan.smem, s);
+    return launch_persist_t<-1, 0>(a, p, false, plan.threads, plan.ctas, plan.smem, s);
 }
 
 namespace {

@@ -254,3 +254,40 @@ def test_gradient_on_device_arrays(ctx, kind, n):
     assert np.all(np.abs(r - ro) <= 2e-4 * np.abs(ro) + 2e-5)
     for k in range(th.shape[0]):
         assert np.max(np.abs(g[k] - go[k])) <= 1e-3 * np.max(np.abs(go[k])) + 1e-12
+
+
+@pytest.mark.parametrize("n_te,dims,pairs", [(12, (19, 16, 9), False), (8, (64, 65, 32), True), (12, (64, 65, 32), True),
+                                             (16, (64, 65, 32), True)])
+@pytest.mark.parametrize("over", [{"convergenceGradTol": 1e-6}, {"convergenceStepTol": 2e-4}, {}])
+def test_tv_pairs_with_statistics(ctx, n_te, dims, pairs, over):
+    """The TV kernel with stopping statistics over several launches of 200
+    epochs, with slices on both sides of the two-voxel variant's rule:
+    parameters equal the per-epoch kernel's bit for bit and the fit
+    stops at the same epoch; the statistics' FP32 sums differ by their order."""
+    import os
+    from gacelle_b200 import phantoms, utils
+    from helpers import run_engine
+    te = np.linspace(2e-3, 40e-3, n_te)
+    mask = phantoms.ellipsoid_mask(dims, 1.05)
+    data, _ = phantoms.r2s_phantom(mask, 5, te=te)
+    idx = utils.mask_index(mask)
+    y = utils.reshape_ND2GD(data, idx)
+    th0 = np.tile(np.array([[1.0], [30.0]], np.float32), (1, y.shape[1]))
+    f = fitting(**dict({"iteration": 410, "lambda": [1e-5], "regmap": ["R2star"], "TVmode": "3D", "patience": 5,
+                        "patienceStep": 5, "patienceGrad": 5, "convergenceStepTol": 1e-12, "convergenceGradTol": 1e-12},
+                       **over))
+    runs = []
+    for kernel in ("persistent", "step"):
+        os.environ["GACELLE_B200_TV_KERNEL"] = kernel
+        try:
+            runs.append(run_engine("r2s", y, th0, f, NAMES["r2s"], dims=mask.shape, gidx=idx.astype(np.int32),
+                                   context=ctx, te=te))
+        finally:
+            del os.environ["GACELLE_B200_TV_KERNEL"]
+    a, b = runs
+    assert bool(a["timing"]["tv_path"] & _lib.TV_PAIRS) == pairs and b["timing"]["tv_path"] == 0
+    assert a["final_niteration"] == b["final_niteration"] and a["stop_reason"] == b["stop_reason"]
+    for k in ("final_theta", "min_theta", "final_residual"):
+        assert np.array_equal(a[k], b[k]), k
+    n = a["final_niteration"] + 1
+    assert np.allclose(a["loss_history"][:n], b["loss_history"][:n], rtol=4e-6, atol=0.0)
