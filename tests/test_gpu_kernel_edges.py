@@ -291,3 +291,30 @@ def test_tv_pairs_with_statistics(ctx, n_te, dims, pairs, over):
         assert np.array_equal(a[k], b[k]), k
     n = a["final_niteration"] + 1
     assert np.allclose(a["loss_history"][:n], b["loss_history"][:n], rtol=4e-6, atol=0.0)
+
+
+@pytest.mark.parametrize("W,steps", [(2, 1), (16, 16), (51, 5), (43, 6), (64, 8), (57, 9), (64, 16), (41, 25), (32, 64),
+                                     (50, 41)])
+@pytest.mark.parametrize("nbin", [2, 1001, 9000])
+def test_posterior_summaries_by_count(ctx, W, steps, nbin):
+    """Median, inter-quartile range and mode of 2 to 2050 samples, around the
+    sorting kernel's sizes (256, 512, 1024, 2048) and with a histogram that does
+    not fit beside its keys (nbin 9000), against the numpy restatement."""
+    from gacelle_b200 import mcmc_solver
+    from gacelle_b200.models import gpuR2starMapping
+    rng = np.random.default_rng(W)
+    te, nv = np.linspace(2e-3, 40e-3, 12), 11
+    m = gpuR2starMapping(te)
+    th = np.vstack([rng.uniform(0.5, 1.5, nv), rng.uniform(10, 60, nv)])
+    y = (th[0] * np.exp(-te[:, None] * th[1]) + 0.02 * rng.standard_normal((12, nv))).astype(np.float32)
+    x0 = np.vstack([th, np.full(nv, 0.02)]).astype(np.float32)
+    lb, ub = list(m.lb[:2]) + [0.02], list(m.ub[:2]) + [0.02]
+    f = mcmc_solver.check_set_default_basic({
+        "algorithm": "GW", "iteration": steps, "thinning": 1, "burnin": 0.0, "Nwalker": W, "lb": lb, "ub": ub, "seed": 3,
+        "Nbin": nbin, "metric": ["median", "iqr", "mode"]})
+    eng = mcmc_solver.mcmc(ctx)._run(m, y, None, x0, None, m.modelParams, f, True, stats=("median", "iqr", "mode"))
+    for k in range(3):
+        med, iqr, mode = oracle.res2out_summaries(eng["posterior"][k].reshape(-1, nv).T, lb[k], ub[k], nbin=nbin)
+        np.testing.assert_array_equal(eng["median"][k], med)
+        np.testing.assert_allclose(eng["iqr"][k], iqr, rtol=1e-6, atol=1e-7)
+        np.testing.assert_array_equal(eng["mode"][k], mode)
