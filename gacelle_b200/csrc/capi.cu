@@ -1886,7 +1886,7 @@ extern "C" gx_status gx_mcmc(gx_context* c, const gx_model* model, int32_t mem, 
         if (post && mcmc_missing_slots(p) > 0) CK(cudaMemsetAsync(post, 0, sizeof(float) * npost, c->stream));
         if (partner) CK(launch_mcmc_partners(p, partner, c->stream));
         int block = o->block_size;
-        if (block == 0 && ng == 0 && autotune_enabled()) TRY(tune_mcmc(c, p, id, &block, &tuned_now));
+        if (block == 0 && ng == 0 && autotune_enabled() && !mcmc_batched(p, id)) TRY(tune_mcmc(c, p, id, &block, &tuned_now));
         block_used = block > 0 ? block : 128;
         float* xstate;
         double* lpstate;

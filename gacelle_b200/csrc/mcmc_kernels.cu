@@ -102,9 +102,11 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
 // the sums are below 2^-21 of their terms: 2^-20 of every term's magnitude
 // plus 2^-20 for every logarithm.  NaN and infinities fail both tests and go
 // to the FP64 form.  Measurements in registers, echo constants in the constant
-// bank.  12,013 voxels x 50 walkers x 500 steps, 12 echoes: 6.93 -> 4.09 ms;
-// Metropolis-Hastings, 4096 voxels x 10,000 steps: 15.4 -> 8.4 ms (one
-// dependent chain a voxel, 1.4-2.1 -> 0.8 us a step).
+// bank; kernels for up to 8, 12 and 16 echoes, since a test per echo and one
+// chain of sums cost a tenth of the kernel.  12,013 voxels x 50 walkers x 500
+// steps, 12 echoes: 6.93 (all FP64) -> 3.65 ms; Metropolis-Hastings, 4096
+// voxels x 10,000 steps: 15.4 -> 6.1 ms (one dependent chain a voxel, 1.4-2.1
+// -> 0.6 us a step).
 constexpr int kScreenM = 16;
 
 struct Screen {
@@ -116,28 +118,25 @@ __device__ __forceinline__ float r2s_residual(float te_l2e, float M0, float R2, 
     return fma1(M0, ex2_ftz(mul1(-te_l2e, R2)), -y);
 }
 
-// P: the protocol in the constant bank (compile-time indices).
+// P: the protocol in the constant bank (compile-time indices); up to MAXM
+// echoes, without a test when the protocol fills the bound.
+template <int MAXM>
 __device__ __forceinline__ Screen screen_eval(const DevProtocol& P, int nm, const float (&x)[3],
-                                              const float (&y)[kScreenM]) {
-    float s = 0.0f;
+                                              const float (&y)[MAXM]) {
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // short chains
+    auto echo = [&](int m) {
+        const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m]);
+        s[m & 3] = fma1(r, r, s[m & 3]);
+    };
+    if (nm == MAXM) {
 #pragma unroll
-    for (int g = 0; g < kScreenM; g += 4) {
-        if (g + 4 <= nm) {
+        for (int m = 0; m < MAXM; ++m) echo(m);
+    } else {
 #pragma unroll
-            for (int m = g; m < g + 4; ++m) {
-                const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m]);
-                s = fma1(r, r, s);
-            }
-        } else {
-#pragma unroll
-            for (int m = g; m < g + 3; ++m)
-                if (m < nm) {
-                    const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m]);
-                    s = fma1(r, r, s);
-                }
-        }
+        for (int m = 0; m < MAXM; ++m)
+            if (m < nm) echo(m);
     }
-    return Screen{s * rcp_ftz(2.0f * x[2] * x[2]), __logf(x[2])};
+    return Screen{((s[0] + s[1]) + (s[2] + s[3])) * rcp_ftz(2.0f * x[2] * x[2]), __logf(x[2])};
 }
 
 // 1 accept, 0 reject, -1 undecided: cz log(zz) + (log p(n) - log p(c)) > log(u)
@@ -148,6 +147,16 @@ __device__ __forceinline__ int screen_decide(int nm, const Screen& c, const Scre
     const float tol = (fm + 20.0f) * 5.9604645e-8f * (c.a + n.a) +
                       9.536743e-7f * (fm * (2.0f + fabsf(c.ln) + fabsf(n.ln)) + fabsf(lz) + fabsf(lu) + cz + 2.0f);
     return d > tol ? 1 : (d < -tol ? 0 : -1);
+}
+
+// The FP64 decision, kept out of line: cz log(zz) + (log p(n) - log p(c)) > log(u).
+__device__ __noinline__ bool exact_accept(const DevProtocol& P, int nm, float c0, float c1, float c2, float n0, float n1,
+                                          float n2, const float* y, int ys, float cz, float zz, float u) {
+    const float xc[3] = {c0, c1, c2}, xn[3] = {n0, n1, n2};
+    VoxAux va{1.0f, nullptr, nullptr, 1};
+    const double lr = (double)cz * (double)logf(zz) +
+                      (log_prob_t<kR2S, 3>(nm, P, xn, y, ys, nullptr, 1, va) - log_prob_t<kR2S, 3>(nm, P, xc, y, ys, nullptr, 1, va));
+    return lr > (double)logf(u);
 }
 
 // Steps k with a kept sample, k > nburnin and (k - nburnin + 1) % thinning
@@ -191,9 +200,10 @@ __device__ __forceinline__ void gw_walker_start(const McmcParams& p, int v, int 
 // keep every per-walker vector in registers; the running sums of the kept
 // samples live in shared memory (each thread its own walkers' slots) and are
 // folded into the per-voxel sums at the end of the launch.
-// SCREEN: acceptance decided by the FP32 screen where it can; the walkers'
-// log-likelihoods are then not kept (xstate determines them).
-template <int MODEL, int NV, bool RB, bool SCREEN>
+// SCREEN > 0: acceptance decided by the FP32 screen where it can (up to SCREEN
+// measurements); the walkers' log-likelihoods are then not kept (xstate
+// determines them).
+template <int MODEL, int NV, bool RB, int SCREEN>
 __global__ void __launch_bounds__(1024, 1)
 gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double* lpstate, double* sum,
           double* sumsq) {
@@ -242,7 +252,7 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
     float x0s[NV], x1s[RB ? NV : 1];
     double lp0 = 0.0, lp1 = 0.0;
     Screen c0{0.0f, 0.0f}, c1{0.0f, 0.0f};
-    float yr[SCREEN ? kScreenM : 1];
+    float yr[SCREEN > 0 ? SCREEN : 1];
 #pragma unroll
     for (int q = 0; q < NV; ++q) x0s[q] = 0.0f;
 #pragma unroll
@@ -273,9 +283,9 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
         }
     }
     __syncthreads();
-    if constexpr (SCREEN) {
+    if constexpr (SCREEN > 0) {
 #pragma unroll
-        for (int m = 0; m < kScreenM; ++m) yr[m] = live && m < nm ? yv[m] : 0.0f;
+        for (int m = 0; m < SCREEN; ++m) yr[m] = live && m < nm ? yv[m] : 0.0f;
         if (own0) c0 = screen_eval(p.P, nm, x0s, yr);
         if constexpr (RB)
             if (own1) c1 = screen_eval(p.P, nm, x1s, yr);
@@ -305,15 +315,11 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
             oob |= (xp < p.lb[j]) || (xp > p.ub[j]);
             xn[j] = fminf(fmaxf(xp, p.lb[j]), p.ub[j]);
         }
-        if constexpr (SCREEN) {
+        if constexpr (SCREEN > 0) {
             cn = screen_eval(p.P, nm, xn, yr);
             int d = screen_decide(nm, cw, cn, (float)(NV - 1), zz, u01(u.y));
-            if (d < 0 && !oob) {
-                const double lr = (double)(NV - 1) * (double)logf(zz) +
-                                  (log_prob_t<MODEL, NV>(nm, s_P, xn, yv, 1, wv, 1, va) -
-                                   log_prob_t<MODEL, NV>(nm, s_P, xw, yv, 1, wv, 1, va));
-                d = lr > (double)logf(u01(u.y));
-            }
+            if (d < 0 && !oob)
+                d = exact_accept(s_P, nm, xw[0], xw[1], xw[2], xn[0], xn[1], xn[2], yv, 1, (float)(NV - 1), zz, u01(u.y));
             return !oob && d > 0;
         }
         lpp = log_prob_t<MODEL, NV>(nm, s_P, xn, yv, 1, wv, 1, va);
@@ -327,7 +333,7 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
             xw[j] = xn[j];
             xv[w * NV + j] = xn[j];
         }
-        if constexpr (SCREEN) cw = cn;
+        if constexpr (SCREEN > 0) cw = cn;
         else lpw = lpp;
         ++nacc;
     };
@@ -382,13 +388,13 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
     if (own0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) xstate[((size_t)q * p.nvox + v) * W + wown0] = x0s[q];
-        if constexpr (!SCREEN) lpstate[(size_t)v * W + wown0] = lp0;
+        if constexpr (SCREEN == 0) lpstate[(size_t)v * W + wown0] = lp0;
     }
     if constexpr (RB) {
         if (own1) {
 #pragma unroll
             for (int q = 0; q < NV; ++q) xstate[((size_t)q * p.nvox + v) * W + wown1] = x1s[q];
-            if constexpr (!SCREEN) lpstate[(size_t)v * W + wown1] = lp1;
+            if constexpr (SCREEN == 0) lpstate[(size_t)v * W + wown1] = lp1;
         }
     }
     if (live) {
@@ -412,7 +418,7 @@ gw_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double*
 // depend on the state, so those of step k + 1 are made while step k's
 // proposal is evaluated: with few voxels a step is one dependent chain, and
 // the draws fill its latencies.
-template <int MODEL, int NV, bool SCREEN>
+template <int MODEL, int NV, int SCREEN>
 __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate,
                           double* lpstate, double* sum, double* sumsq) {
     __shared__ DevProtocol s_P;
@@ -434,7 +440,7 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
     float x[NV];
     double lp = 0.0;
     Screen cs{0.0f, 0.0f};
-    float yr[SCREEN ? kScreenM : 1];
+    float yr[SCREEN > 0 ? SCREEN : 1];
     double s1[NV], s2[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) { s1[q] = 0.0; s2[q] = 0.0; x[q] = 0.0f; }
@@ -456,15 +462,15 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
 #pragma unroll
             for (int q = 0; q < NV; ++q)
                 x[q] = fminf(fmaxf(p.x0[(size_t)q * p.nvox + v], p.lb[q]), p.ub[q]);
-            if constexpr (!SCREEN) lp = log_prob_t<MODEL, NV>(nm, s_P, x, yv, p.nvox, wv, p.nvox, va);
+            if constexpr (SCREEN == 0) lp = log_prob_t<MODEL, NV>(nm, s_P, x, yv, p.nvox, wv, p.nvox, va);
         } else {
 #pragma unroll
             for (int q = 0; q < NV; ++q) x[q] = xstate[(size_t)q * p.nvox + v];
-            if constexpr (!SCREEN) lp = lpstate[v];
+            if constexpr (SCREEN == 0) lp = lpstate[v];
         }
-        if constexpr (SCREEN) {
+        if constexpr (SCREEN > 0) {
 #pragma unroll
-            for (int m = 0; m < kScreenM; ++m) yr[m] = m < nm ? yv[(size_t)m * p.nvox] : 0.0f;
+            for (int m = 0; m < SCREEN; ++m) yr[m] = m < nm ? yv[(size_t)m * p.nvox] : 0.0f;
             cs = screen_eval(p.P, nm, x, yr);
         }
         int kept_k = first_kept(p, k0);
@@ -481,13 +487,12 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
             }
             const float uk = u;
             bool acc;
-            if constexpr (SCREEN) {
+            if constexpr (SCREEN > 0) {
                 const Screen cp = screen_eval(p.P, nm, xp, yr);
                 draws(k + 1, nrm, u);
                 int d = screen_decide(nm, cs, cp, 0.0f, 1.0f, uk);
                 if (d < 0 && !oob)
-                    d = (log_prob_t<MODEL, NV>(nm, s_P, xp, yv, p.nvox, wv, p.nvox, va) -
-                         log_prob_t<MODEL, NV>(nm, s_P, x, yv, p.nvox, wv, p.nvox, va)) > (double)logf(uk);
+                    d = exact_accept(s_P, nm, x[0], x[1], x[2], xp[0], xp[1], xp[2], yv, p.nvox, 0.0f, 1.0f, uk);
                 acc = !oob && d > 0;
                 if (acc) cs = cp;
             } else {
@@ -517,7 +522,7 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
         }
 #pragma unroll
         for (int q = 0; q < NV; ++q) xstate[(size_t)q * p.nvox + v] = x[q];
-        if constexpr (!SCREEN) lpstate[v] = lp;
+        if constexpr (SCREEN == 0) lpstate[v] = lp;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             sum[(size_t)j * p.nvox + v] += s1[j];
@@ -527,6 +532,128 @@ __global__ void mh_kernel(McmcParams p, int rr, int k0, int k1, int init, float*
     unsigned int wsum = nacc;
     for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
     if ((threadIdx.x & 31) == 0 && wsum) atomicAdd(p.n_acc, (unsigned long long)wsum);
+}
+
+// ---------------------------------------------------------------------------
+// Metropolis-Hastings for few voxels (screened R2*).  With a warp or less a
+// scheduler a chain is bound by its own latencies, and half of a step's
+// instructions are its draws, which no state enters.  A CTA takes 32 voxels:
+// warps 1-3 make the draws of the next kMhBatch steps into one of two shared
+// buffers while warp 0 runs the chains through the other, one barrier a batch.
+// Same draws, same decisions as mh_kernel.  Seven drawing warps measured
+// slower (2.8 against 2.6 ms below).
+// Whole call, 12 echoes, mh_kernel -> this one: 1000 voxels x 10,000 steps
+// 5.9 -> 2.3 ms, 4096 x 10,000 6.25 -> 2.6, 10,000 x 10,000 6.6 -> 3.8,
+// 20,000 x 4000 4.25 -> 3.55, 40,000 x 3000 6.64 -> 6.70: six chain warps an
+// SM are the line; beyond, the chains fill each other's latencies anyway.
+// ---------------------------------------------------------------------------
+constexpr int kMhBatch = 16;
+constexpr int kMhBatchVoxels = 148 * 6 * 32;
+
+template <int MAXM>
+__global__ void __launch_bounds__(128)
+mh_batch_kernel(McmcParams p, int rr, int k0, int k1, int init, float* xstate, double* sum, double* sumsq) {
+    constexpr int NV = 3;
+    __shared__ DevProtocol s_P;
+    __shared__ float4 s_draw[2][kMhBatch][32];  // three normals, the acceptance uniform
+    stage_protocol(p.P, &s_P);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int v = blockIdx.x * 32 + lane;
+    const bool live = v < p.nvox;
+    const int nm = p.nm;
+    auto make = [&](int first, float4 (*buf)[32]) {  // steps first, first + 1, .. of a batch, by warps 1-3
+        const uint32_t tag = kTagMhMove | ((uint32_t)rr << 16);
+        for (int i = warp - 1; i < kMhBatch && first + i <= k1; i += 3) {
+            const uint32_t k = (uint32_t)(first + i);
+            const U4 r = philox((uint32_t)v, k, 0u, tag, p.seed);
+            float n0, n1, n2, n3;
+            box_muller(r.x, r.y, n0, n1);
+            box_muller(r.z, r.w, n2, n3);
+            buf[i][lane] = make_float4(n0, n1, n2, u01(philox((uint32_t)v, k, 8u, tag, p.seed).x));
+        }
+    };
+    float x[NV], yr[MAXM];
+    double s1[NV], s2[NV];
+    Screen cs{0.0f, 0.0f};
+    unsigned int nacc = 0;
+    int kept_k = 0;
+    const float* yv = p.data + (live ? v : 0);
+    if (warp == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            s1[q] = s2[q] = 0.0;
+            // a lane without a voxel runs along on a harmless state and writes nothing
+            x[q] = !live ? 1.0f
+                   : init ? fminf(fmaxf(p.x0[(size_t)q * p.nvox + v], p.lb[q]), p.ub[q])
+                          : xstate[(size_t)q * p.nvox + v];
+        }
+#pragma unroll
+        for (int m = 0; m < MAXM; ++m) yr[m] = m < nm ? yv[(size_t)m * p.nvox] : 0.0f;
+        cs = screen_eval(p.P, nm, x, yr);
+        kept_k = first_kept(p, k0);
+    } else {
+        make(k0, s_draw[0]);
+    }
+    __syncthreads();
+    for (int kb = k0, b = 0; kb <= k1; kb += kMhBatch, b ^= 1) {
+        if (warp > 0) {
+            make(kb + kMhBatch, s_draw[b ^ 1]);
+        } else {
+            const int n = min(kMhBatch, k1 - kb + 1);
+            float4 d = s_draw[b][0][lane];
+            for (int i = 0; i < n; ++i) {
+                const float4 dn = s_draw[b][min(i + 1, n - 1)][lane];
+                const float nrm[NV] = {d.x, d.y, d.z}, uk = d.w;
+                float xp[NV];
+                bool oob = false;
+#pragma unroll
+                for (int q = 0; q < NV; ++q) {
+                    float t = x[q] + p.xstep[q] * nrm[q];
+                    oob |= (t < p.lb[q]) || (t > p.ub[q]);
+                    xp[q] = fminf(fmaxf(t, p.lb[q]), p.ub[q]);
+                }
+                const Screen cp = screen_eval(p.P, nm, xp, yr);
+                int dec = screen_decide(nm, cs, cp, 0.0f, 1.0f, uk);
+                if (dec < 0 && !oob && live)
+                    dec = exact_accept(s_P, nm, x[0], x[1], x[2], xp[0], xp[1], xp[2], yv, p.nvox, 0.0f, 1.0f, uk);
+                const bool acc = !oob && dec > 0;
+                if (acc) {
+                    cs = cp;
+                    ++nacc;
+                }
+#pragma unroll
+                for (int q = 0; q < NV; ++q) x[q] = acc ? xp[q] : x[q];
+                if (kb + i == kept_k) {
+                    kept_k += p.thinning;
+                    const int c = kept_index(p, kb + i);
+                    if (c >= 0 && live)
+#pragma unroll
+                        for (int j = 0; j < NV; ++j) {
+                            double e = (double)x[j] - (double)p.shift[(size_t)j * p.nvox + v];
+                            s1[j] += e;
+                            s2[j] += e * e;
+                            if (p.posterior)
+                                p.posterior[(((size_t)j * p.repetition + rr) * p.ns + c) * p.nvox + v] = x[j];
+                        }
+                }
+                d = dn;
+            }
+        }
+        __syncthreads();
+    }
+    if (warp > 0) return;
+    if (live) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            xstate[(size_t)q * p.nvox + v] = x[q];
+            sum[(size_t)q * p.nvox + v] += s1[q];
+            sumsq[(size_t)q * p.nvox + v] += s2[q];
+        }
+    } else {
+        nacc = 0;
+    }
+    for (int o = 16; o > 0; o >>= 1) nacc += __shfl_xor_sync(0xffffffffu, nacc, o);
+    if (lane == 0 && nacc) atomicAdd(p.n_acc, (unsigned long long)nacc);
 }
 
 // ---------------------------------------------------------------------------
@@ -905,6 +1032,10 @@ static void gw_shape(const McmcParams& p, int block_hint, int* vpb, int* block, 
 // measurements are held in registers.
 static bool screened(const McmcParams& p) { return p.weights == nullptr && p.nm <= kScreenM; }
 
+bool mcmc_batched(const McmcParams& p, int model) {
+    return p.algorithm == 0 && model == kR2S && screened(p) && p.nvox <= kMhBatchVoxels;
+}
+
 // Steps [k0, k1] of repetition rr as one launch (init: the walkers start at k0 == 1).
 template <int MODEL>
 static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k0, int k1, float* xstate,
@@ -916,9 +1047,12 @@ static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k
         size_t smem;
         gw_shape(p, block_hint, &vpb, &block, &smem);
         const int nb = (p.nvox + vpb - 1) / vpb;
-        auto k = p.update == 0 ? gw_kernel<MODEL, NV, false, false> : gw_kernel<MODEL, NV, true, false>;
+        auto k = p.update == 0 ? gw_kernel<MODEL, NV, false, 0> : gw_kernel<MODEL, NV, true, 0>;
         if constexpr (MODEL == kR2S)
-            if (screened(p)) k = p.update == 0 ? gw_kernel<MODEL, NV, false, true> : gw_kernel<MODEL, NV, true, true>;
+            if (screened(p))
+                k = p.nm <= 8    ? (p.update == 0 ? gw_kernel<MODEL, NV, false, 8> : gw_kernel<MODEL, NV, true, 8>)
+                    : p.nm <= 12 ? (p.update == 0 ? gw_kernel<MODEL, NV, false, 12> : gw_kernel<MODEL, NV, true, 12>)
+                                 : (p.update == 0 ? gw_kernel<MODEL, NV, false, 16> : gw_kernel<MODEL, NV, true, 16>);
         if (kIsNexi<MODEL>) p.node_smem = nodes_fit(&smem);
         if (smem + sizeof(DevProtocol) > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -928,9 +1062,16 @@ static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k
     } else {
         const int block = block_hint > 0 ? block_hint : 128;
         const int nb = (p.nvox + block - 1) / block;
-        auto k = mh_kernel<MODEL, NV, false>;
-        if constexpr (MODEL == kR2S)
-            if (screened(p)) k = mh_kernel<MODEL, NV, true>;
+        auto k = mh_kernel<MODEL, NV, 0>;
+        if constexpr (MODEL == kR2S) {
+            if (block_hint <= 0 && mcmc_batched(p, MODEL)) {
+                auto kb = p.nm <= 8 ? mh_batch_kernel<8> : p.nm <= 12 ? mh_batch_kernel<12> : mh_batch_kernel<16>;
+                kb<<<(p.nvox + 31) / 32, 128, 0, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, sum, sumsq);
+                ++g_kernel_launches;
+                return cudaGetLastError();
+            }
+            if (screened(p)) k = p.nm <= 8 ? mh_kernel<MODEL, NV, 8> : p.nm <= 12 ? mh_kernel<MODEL, NV, 12> : mh_kernel<MODEL, NV, 16>;
+        }
         k<<<nb, block, 0, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, lpstate, sum, sumsq);
     }
     ++g_kernel_launches;

@@ -85,6 +85,31 @@ def test_r2s_chain_decisions(ctx, update, n_te):
     assert np.mean(np.abs(pe - po) <= 1e-4 * np.abs(po) + 1e-7) > 0.97
 
 
+@pytest.mark.parametrize("n_te,nvox,steps", [(1, 1, 15), (8, 31, 16), (9, 33, 17), (12, 32, 33), (13, 64, 1),
+                                             (16, 65, 160)])
+def test_mh_batched_draws(ctx, n_te, nvox, steps):
+    """The kernel whose draws are made ahead by other warps takes the moves of
+    the plain one (a chosen block size), bit for bit: same draws and same
+    decisions.  Steps around a batch of 16, voxels around a warp, echoes around
+    the kernels' bounds."""
+    from gacelle_b200 import mcmc_solver
+    from gacelle_b200.models import gpuR2starMapping
+    rng = np.random.default_rng(n_te + steps)
+    te = np.linspace(2e-3, 40e-3, n_te)
+    m = gpuR2starMapping(te)
+    th = np.vstack([rng.uniform(0.5, 1.5, nvox), rng.uniform(10, 60, nvox)])
+    y = (th[0] * np.exp(-te[:, None] * th[1]) + 0.02 * rng.standard_normal((n_te, nvox))).astype(np.float32)
+    x0 = np.vstack([th, np.full(nvox, 0.02)]).astype(np.float32)
+    out = []
+    for block in (0, 64):
+        f = mcmc_solver.check_set_default_basic({
+            "algorithm": "MH", "iteration": steps, "thinning": 1, "burnin": 0.0, "lb": m.lb, "ub": m.ub,
+            "xStepSize": m.step, "seed": 4, "repetition": 2, "blockSize": block})
+        out.append(mcmc_solver.mcmc(ctx)._run(m, y, None, x0, None, m.modelParams, f, True))
+    for key in ("posterior", "mean", "std"):
+        assert np.array_equal(out[0][key], out[1][key], equal_nan=True), key
+
+
 @pytest.mark.parametrize("n_te", [20, 22, 23, 24])
 def test_block_near_the_default_shared_memory_limit(ctx, n_te):
     """A 512-thread block whose measurements and staged protocol lie around
