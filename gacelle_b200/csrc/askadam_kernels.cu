@@ -19,6 +19,7 @@
 // Reference: utils/askadam.m (model_gradient :23-117, optimisation :121-365,
 // initialise_parameter :368-412, update_parameters :673-691,
 // unscale_parameters :1063-1075), utils/spatial_total_variation.m.
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 
@@ -133,6 +134,91 @@ __global__ void init_state_kernel(AdamParams a, const float* theta0, float rando
 // ---------------------------------------------------------------------------
 // Fused multi-epoch kernel (no spatial coupling).
 // ---------------------------------------------------------------------------
+// One evaluation of voxel v: the gradient gz with respect to its unconstrained
+// parameters z, and the history's quantities q (loss; with STATS also the
+// regulariser, |gz|^2, |z|^2, |z - zp|^2).  y, w: its measurements and weights,
+// ys apart; res: its residual row or nullptr.
+template <int MODEL, int LOSS, bool STATS>
+__device__ __forceinline__ void fused_eval(const AdamParams& a, const DevProtocol& P, const DevVol& V, int v, bool valid,
+                                           const VoxAux& va, const LossAux& aux, const float* y, const float* w, int ys,
+                                           float* res, const float (&z)[ModelNP<MODEL>::value],
+                                           const float (&zp)[ModelNP<MODEL>::value],
+                                           float (&gz)[ModelNP<MODEL>::value], float (&q)[STATS ? kHistW : 1]) {
+    constexpr int NP = ModelNP<MODEL>::value;
+    constexpr int NQ = STATS ? kHistW : 1;
+    const float normf = V.norm;
+    float th[NP], dth[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) th[k] = unscale(a.transform, a.P.lb[k], a.P.ub[k], z[k], dth[k]);
+    LossAcc<LOSS, NP> acc;
+    acc.total = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) acc.g[k] = 0.0f;
+    acc.y = y; acc.ys = ys;
+    acc.w = w; acc.ws = ys;
+    acc.aux = aux; acc.mse_scale = a.mse_scale; acc.hd = a.huber_delta;
+    acc.res = res;
+    acc.rs = a.nvtot;
+    model_eval<MODEL, MODEL == kR1R2S>(P, th, va, acc);
+    acc.finish();
+    float reg = 0.0f;
+    if (a.prior_mu) {  // prior regulariser (the host records it through STATS)
+        float gth[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) gth[k] = acc.g[k] * normf;
+        if (valid) prior_voxel<NP>(a, V, v, th, gth, reg);
+#pragma unroll
+        for (int k = 0; k < NP; ++k) gz[k] = gth[k] * dth[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) gz[k] = acc.g[k] * normf * dth[k];
+    }
+    q[0] = valid ? acc.total : 0.0f;
+    if (STATS) {
+        float g2 = 0.f, z2 = 0.f, d2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            g2 += gz[k] * gz[k];
+            z2 += z[k] * z[k];
+            d2 += (z[k] - zp[k]) * (z[k] - zp[k]);
+        }
+        q[NQ > 1 ? 1 : 0] = reg;
+        if (NQ > 4) {
+            q[2] = valid ? g2 : 0.f;
+            q[3] = valid ? z2 : 0.f;
+            q[4] = valid ? d2 : 0.f;
+        }
+    }
+}
+
+// First checkpoint epoch (a multiple of ckpt_every) from e_begin on.
+__device__ __forceinline__ int first_checkpoint(const AdamParams& a, int e_begin) {
+    return a.ckpt_every > 0 ? (e_begin + a.ckpt_every - 1) / a.ckpt_every * a.ckpt_every : INT_MAX;
+}
+
+// The update after epoch e, and its checkpoint when it is due.
+template <int NP, bool STATS>
+__device__ __forceinline__ void fused_step(const AdamParams& a, int v, bool valid, int e, int& next_ck, float (&z)[NP],
+                                           float (&m1)[NP], float (&m2)[NP], float (&zp)[NP], const float (&gz)[NP]) {
+    const float2 sc = a.sched[e];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        if (STATS) zp[k] = z[k];
+        opt_update(a, sc, z[k], m1[k], m2[k], gz[k]);
+    }
+    if (e == next_ck) {
+        next_ck += a.ckpt_every;
+        float* c = a.ckpt + (size_t)(e / a.ckpt_every) * ((size_t)3 * NP * a.nvtot);
+        if (valid)
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                c[(size_t)k * a.nvtot + v] = z[k];
+                c[(size_t)(NP + k) * a.nvtot + v] = m1[k];
+                c[(size_t)(2 * NP + k) * a.nvtot + v] = m2[k];
+            }
+    }
+}
+
 template <int MODEL, int LOSS, bool STATS>
 __device__ __forceinline__ void fused_body(const AdamParams& a, int e_begin, int e_end, int update_last, int record) {
     constexpr int NP = ModelNP<MODEL>::value;
@@ -177,80 +263,16 @@ __device__ __forceinline__ void fused_body(const AdamParams& a, int e_begin, int
         m2[k] = a.m2[i];
         zp[k] = STATS ? a.zprev[i] : 0.0f;
     }
-    const float normf = V.norm;
     const double normd = V.normd;
-    const size_t slot = (size_t)3 * NP * a.nvtot;
-    // the next checkpoint epoch (a multiple of ckpt_every), kept as a counter
-    int next_ck = a.ckpt_every > 0 ? (e_begin + a.ckpt_every - 1) / a.ckpt_every * a.ckpt_every : INT_MAX;
+    int next_ck = first_checkpoint(a, e_begin);
 
     for (int e = e_begin; e <= e_end; ++e) {
-        float th[NP], dth[NP];
-#pragma unroll
-        for (int k = 0; k < NP; ++k) th[k] = unscale(a.transform, a.P.lb[k], a.P.ub[k], z[k], dth[k]);
-        LossAcc<LOSS, NP> acc;
-        acc.total = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NP; ++k) acc.g[k] = 0.0f;
-        acc.y = s_y + tid; acc.ys = B;
-        acc.w = a.weights ? s_w + tid : nullptr; acc.ws = B;
-        acc.aux = aux; acc.mse_scale = a.mse_scale; acc.hd = a.huber_delta;
-        acc.res = (a.res_out && e == e_end && valid) ? a.res_out + v : nullptr;
-        acc.rs = a.nvtot;
-        model_eval<MODEL, MODEL == kR1R2S>(s_P, th, va, acc);
-        acc.finish();
-        float gz[NP];
-        float reg = 0.0f;
-        if (a.prior_mu) {  // prior regulariser (the host records it through STATS)
-            float gth[NP];
-#pragma unroll
-            for (int k = 0; k < NP; ++k) gth[k] = acc.g[k] * normf;
-            if (valid) prior_voxel<NP>(a, V, v, th, gth, reg);
-#pragma unroll
-            for (int k = 0; k < NP; ++k) gz[k] = gth[k] * dth[k];
-        } else {
-#pragma unroll
-            for (int k = 0; k < NP; ++k) gz[k] = acc.g[k] * normf * dth[k];
-        }
-        if (record) {
-            float q[NQ];
-            q[0] = valid ? acc.total : 0.0f;
-            if (STATS) {
-                float g2 = 0.f, z2 = 0.f, d2 = 0.f;
-#pragma unroll
-                for (int k = 0; k < NP; ++k) {
-                    g2 += gz[k] * gz[k];
-                    z2 += z[k] * z[k];
-                    d2 += (z[k] - zp[k]) * (z[k] - zp[k]);
-                }
-                q[NQ > 1 ? 1 : 0] = reg;
-                if (NQ > 4) {
-                    q[2] = valid ? g2 : 0.f;
-                    q[3] = valid ? z2 : 0.f;
-                    q[4] = valid ? d2 : 0.f;
-                }
-            }
-            block_accumulate<NQ>(q, a.hist + ((size_t)vol * (a.niter + 1) + e) * kHistW, normd,
-                                 s_red, e & 1);
-        }
-        if (e <= update_last) {
-            float2 sc = a.sched[e];
-#pragma unroll
-            for (int k = 0; k < NP; ++k) {
-                if (STATS) zp[k] = z[k];
-                opt_update(a, sc, z[k], m1[k], m2[k], gz[k]);
-            }
-            if (e == next_ck) {
-                next_ck += a.ckpt_every;
-                float* c = a.ckpt + (size_t)(e / a.ckpt_every) * slot;
-                if (valid)
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) {
-                        c[(size_t)k * a.nvtot + v] = z[k];
-                        c[(size_t)(NP + k) * a.nvtot + v] = m1[k];
-                        c[(size_t)(2 * NP + k) * a.nvtot + v] = m2[k];
-                    }
-            }
-        }
+        float gz[NP], q[NQ];
+        fused_eval<MODEL, LOSS, STATS>(a, s_P, V, v, valid, va, aux, s_y + tid, a.weights ? s_w + tid : nullptr, B,
+                                       a.res_out && e == e_end && valid ? a.res_out + v : nullptr, z, zp, gz, q);
+        if (record)
+            block_accumulate<NQ>(q, a.hist + ((size_t)vol * (a.niter + 1) + e) * kHistW, normd, s_red, e & 1);
+        if (e <= update_last) fused_step<NP, STATS>(a, v, valid, e, next_ck, z, m1, m2, zp, gz);
     }
     if (valid) {
 #pragma unroll
@@ -280,11 +302,120 @@ __global__ void __maxnreg__(80) fused_kernel_r1r2s(AdamParams a, int e_begin, in
 
 // NEXI with lmax 0: registers capped at 96 (20 warps an SM; uncapped up to
 // 128, 16 warps): 328,050 voxels x 14 nodes, MSE, 195 -> 187 us an iteration,
-// 100,003 voxels x 100 nodes, Rician loss, 429 -> 414 us; 88 and 80 are slower
-// again.  lmax 2 keeps twice the sums and would spill.
+// 100,003 voxels x 100 nodes, Rician loss, 429 -> 414 us (179 and 403 since the
+// node loop carries its partial results negated); 88 and 80 are slower again.
+// lmax 2 keeps twice the sums and would spill.
 template <int MODEL, int LOSS, bool STATS>
 __global__ void __maxnreg__(96) fused_kernel_nexi(AdamParams a, int e_begin, int e_end, int update_last, int record) {
     fused_body<MODEL, LOSS, STATS>(a, e_begin, e_end, update_last, record);
+}
+
+// ---------------------------------------------------------------------------
+// NEXI with lmax 0 when the voxels fill the resident warps a few times: the
+// blocks of fused_kernel_nexi run all epochs of their voxels, so a last wave
+// with few blocks (100,003 voxels: 44 of 784) costs its whole latency-bound
+// run.  Here one CTA an SM owns a share of the work-list, in tasks of 32
+// voxels, and its 20 warps take (task, epochs) units in turn: unit i is task
+// i % n, epochs i / n, by warp i % 20, so the warps stay busy until the last
+// round.  Between units a task's state lives in global memory; a unit waits for
+// the task's previous one (n units earlier, n > 20, of a warp of the same CTA:
+// the least unfinished unit never waits, so all end), with a limit on the wait.
+// Per voxel the operations of fused_kernel_nexi.  24 warps at 80 registers: 0-2 %
+// slower or faster by size, and from 25 tasks on only.
+// ---------------------------------------------------------------------------
+constexpr int kRotWarps = 20;              // 640 threads x 96 registers
+constexpr int kRotTasks = 96;              // tasks of a CTA, at most
+constexpr long long kRotWait = 1LL << 32;  // clocks, about 2 s
+
+template <int LOSS, bool STATS>
+__global__ void __maxnreg__(96) fused_kernel_nexi_turns(AdamParams a, int e_begin, int e_end, int update_last, int record,
+                                                        int block, int span) {
+    constexpr int MODEL = kNEXI, NP = ModelNP<MODEL>::value, NQ = STATS ? kHistW : 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ DevProtocol s_P;
+    __shared__ volatile int s_done[kRotTasks];  // spans finished of a task
+    __shared__ volatile int s_err;
+    NexiNodes* s_nodes = reinterpret_cast<NexiNodes*>(smem_raw);
+    float* s_y = reinterpret_cast<float*>(s_nodes + 1);
+    const int B = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* s_w = s_y + a.nm * B;
+    const int ntask = a.nvtot / 32;
+    const int t0 = (int)((long long)blockIdx.x * ntask / gridDim.x);
+    const int n = (int)((long long)(blockIdx.x + 1) * ntask / gridDim.x) - t0;
+    stage_protocol(a.P, &s_P);
+    stage_nodes(a.nodes, s_nodes);
+    for (int i = tid; i < n; i += B) s_done[i] = 0;
+    if (tid == 0) s_err = 0;
+    __syncthreads();
+    const int nspan = (e_end - e_begin + span) / span;
+    for (int u = warp; u < n * nspan; u += kRotWarps) {
+        const int t = u % n, c = u / n;
+        if (c > 0) {
+            int bad = 0;
+            if (lane == 0) {
+                const long long start = clock64();
+                while (s_done[t] < c && !bad) {
+                    __nanosleep(64);
+                    bad = s_err || clock64() - start > kRotWait;
+                }
+                if (bad) {
+                    s_err = 1;
+                    *a.wait_err = 1;
+                }
+            }
+            if (__shfl_sync(0xffffffffu, bad, 0)) return;
+            __threadfence();
+        }
+        const int v = (t0 + t) * 32 + lane;
+        const int vol = a.blk_vol[(t0 + t) * 32 / block];
+        const DevVol& V = a.vols[vol];
+        const bool valid = (v - V.off) < V.nvox;
+        for (int m = 0; m < a.nm; ++m) s_y[m * B + tid] = a.data[(size_t)m * a.nvtot + v];
+        if (a.weights)
+            for (int m = 0; m < a.nm; ++m) s_w[m * B + tid] = a.weights[(size_t)m * a.nvtot + v];
+        VoxAux va{1.0f, nullptr, nullptr, B};
+        va.sigma = voxel_sigma(a, v);
+        va.nodes = s_nodes;
+        const LossAux aux = make_loss_aux(va.sigma);
+        float z[NP], m1[NP], m2[NP], zp[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {  // from L2: another warp's stores
+            const size_t i = (size_t)k * a.nvtot + v;
+            z[k] = __ldcg(a.z + i);
+            m1[k] = __ldcg(a.m1 + i);
+            m2[k] = __ldcg(a.m2 + i);
+            zp[k] = STATS ? __ldcg(a.zprev + i) : 0.0f;
+        }
+        const int eb = e_begin + c * span, ee = min(eb + span - 1, e_end);
+        int next_ck = first_checkpoint(a, eb);
+        for (int e = eb; e <= ee; ++e) {
+            float gz[NP], q[NQ];
+            fused_eval<MODEL, LOSS, STATS>(a, s_P, V, v, valid, va, aux, s_y + tid, a.weights ? s_w + tid : nullptr, B,
+                                           a.res_out && e == e_end && valid ? a.res_out + v : nullptr, z, zp, gz, q);
+            if (record) {
+                double* h = a.hist + ((size_t)vol * (a.niter + 1) + e) * kHistW;
+#pragma unroll
+                for (int k = 0; k < NQ; ++k) {
+                    const double s = (double)warp_sum(q[k]) * (k == 0 ? V.normd : 1.0);
+                    if (lane == 0 && s != 0.0) atomicAdd(h + k, s);
+                }
+            }
+            if (e <= update_last) fused_step<NP, STATS>(a, v, valid, e, next_ck, z, m1, m2, zp, gz);
+        }
+        if (valid) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                const size_t i = (size_t)k * a.nvtot + v;
+                a.z[i] = z[k];
+                a.m1[i] = m1[k];
+                a.m2[i] = m2[k];
+                if (STATS) a.zprev[i] = zp[k];
+            }
+        }
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) s_done[t] = c + 1;
+    }
 }
 
 template <int MODEL, int LOSS, bool STATS>
@@ -986,12 +1117,56 @@ int nodes_fit(size_t* smem) {
     return 1;
 }
 
+// Multiprocessors of the current device (0 on error).
+int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return n;
+}
+
+// Whether fused_kernel_nexi_turns may take a work-list: more than 20 tasks an SM
+// (fewer are resident at once anyway) and at most 96, beyond which a partial
+// wave of the block kernel weighs less than the turns' reloads.  Block kernel
+// -> turns, whole calls: 100,003 voxels x 100 nodes, Rician, 40 epochs (22
+// tasks) 16.3 -> 14.2 ms; 14 nodes, MSE, 100 epochs: 100,000 voxels 6.64 ->
+// 5.74, 150,000 8.29 -> 8.19, 328,050 (70 tasks) 18.2 -> 17.6; 640,000 voxels x
+// 60 epochs (136 tasks) 20.3 -> 20.6.
+bool nexi_turns(int nvtot, int nsm) {
+    const int ntask = nvtot / 32;
+    return nsm > 0 && ntask / nsm > kRotWarps && (ntask + nsm - 1) / nsm <= kRotTasks;
+}
+
+// Epochs of a unit of fused_kernel_nexi_turns (about 32 rounds a launch, for a
+// small last one), or 0: not for this launch.
+static int nexi_span(const AdamParams& a, int e_begin, int e_end, int nvox, int nsm, size_t* smem) {
+    *smem = sizeof(NexiNodes) + sizeof(float) * (size_t)(32 * kRotWarps) * a.nm * (a.weights ? 2 : 1);
+    const int epochs = e_end - e_begin + 1;
+    if (!a.wait_err || nvox != a.nvtot || !nexi_turns(nvox, nsm) || epochs < 2 || a.P.nx > kNodeTab ||
+        *smem + sizeof(DevProtocol) + 1024 > kMaxSmemPerBlock)
+        return 0;
+    return std::max(1, (int)((long long)((nvox / 32 + nsm - 1) / nsm) * epochs / (32 * kRotWarps)));
+}
+
 template <int MODEL, int LOSS, bool STATS>
 static cudaError_t fused_dispatch3(AdamParams a, int e_begin, int e_end, int update_last,
                                    bool record, int block, int nblocks, cudaStream_t s) {
     constexpr int NQ = STATS ? kHistW : 1;
     size_t smem = sizeof(double) * 2 * 32 * NQ +
                   sizeof(float) * (size_t)block * (a.nm * (a.weights ? 2 : 1) + 2 * a.P.n_fa);
+    if constexpr (MODEL == kNEXI) {
+        size_t turns;
+        const int nsm = a.wait_err ? sm_count() : 0;
+        const int span = nexi_span(a, e_begin, e_end, block * nblocks, nsm, &turns);
+        if (span > 0) {
+            auto kt = fused_kernel_nexi_turns<LOSS, STATS>;
+            const cudaError_t err = cudaFuncSetAttribute(kt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)turns);
+            if (err != cudaSuccess) return err;
+            kt<<<nsm, 32 * kRotWarps, turns, s>>>(a, e_begin, e_end, update_last, record ? 1 : 0, block, span);
+            ++g_kernel_launches;
+            return cudaGetLastError();
+        }
+    }
     auto k = fused_kernel_fn<MODEL, LOSS, STATS>();
     if (kIsNexi<MODEL>) a.node_smem = nodes_fit(&smem);
     if (smem + sizeof(DevProtocol) > 48 * 1024) {

@@ -91,7 +91,7 @@ enum Slot {
     S_MC_PART, S_MC_SUM, S_MC_SUMSQ, S_MC_SHIFT, S_MC_X0, S_MC_POST, S_MC_ACC, S_MC_MEAN,
     S_MC_STD, S_FWD_TH, S_FWD_SIG, S_FWD_B1, S_BAR, S_MC_GLOB, S_ROBUST, S_DICT_SIG, S_DICT_D,
     S_DICT_W, S_DICT_OP, S_DICT_LIST, S_DICT_STAT, S_DICT_E, S_DICT_C, S_DICT_B, S_DICT_S, S_FLAGS, S_DATA_QUADS, S_PRIOR_MU, S_PRIOR_SD, S_SURF_NB, S_SURF_LEN,
-    S_MC_STATS, S_MC_X, S_MC_LP, S_TUNE, S_TUNE_HIST, S_BLK_L, S_HGRID0, S_HGRID1, S_NSLOTS
+    S_MC_STATS, S_MC_X, S_MC_LP, S_TUNE, S_TUNE_HIST, S_BLK_L, S_WAIT_ERR, S_HGRID0, S_HGRID1, S_NSLOTS
 };
 
 struct gx_context {
@@ -1003,6 +1003,7 @@ static gx_status replay_volume(AdamJob& J, int i, int target, float* th_out, flo
     AdamParams base = J.a;
     base.z = J.zr; base.m1 = J.m1r; base.m2 = J.m2r;
     base.zprev = nullptr;
+    base.wait_err = nullptr;
     base.ckpt_every = 0;
     View V;
     TRY(make_view(J, i, base, &V));
@@ -1147,6 +1148,10 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
     const bool stop_possible = can_stop(o);
     const int chunk = stop_possible ? (o->chunk > 0 ? o->chunk : 200) : (N > 0 ? N : 1);
     TRY(alloc_outputs(J, out));
+    if (!J.tv && J.id == kNEXI && nexi_turns(J.nvtot, sm_count())) {
+        TRY(wsT(c, S_WAIT_ERR, 1, &J.a.wait_err));
+        CK(cudaMemsetAsync(J.a.wait_err, 0, sizeof(int), c->stream));
+    }
     if (J.autotune) TRY(tune_fused(J));
     if (J.tv) {
         const char* env = getenv("GACELLE_B200_TV_KERNEL");
@@ -1248,6 +1253,12 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
         PersistBarrier hb;
         CK(cudaMemcpy(&hb, J.barrier, sizeof(hb), cudaMemcpyDeviceToHost));
         if (hb.error) return fail(GX_ETIMEOUT, "askAdam TV kernel: a grid barrier wait expired");
+    }
+    if (J.a.wait_err) {
+        int expired = 0;
+        CK(cudaMemcpyAsync(&expired, J.a.wait_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        if (expired) return fail(GX_ETIMEOUT, "askAdam fused kernel: a wait expired");
     }
     for (int i = 0; i < J.nvol && N > 0; ++i) {  // the initial evaluation equals epoch 1's
         size_t base = (size_t)i * (N + 1) * kHistW;

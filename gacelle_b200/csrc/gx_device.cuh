@@ -682,6 +682,9 @@ GX_HD void nexi_node(int nx, float h, int i, float2& x2, float2& w, float2& wx2,
 // 28, but their combinations cancel, and the sums' rounding made d/dra and
 // d/dDe 4-10 times less exact; dM/dd2 and dM/dr1 as differences of the other
 // two, or from (r1 + r2 -+ (d2 - d1)) W - a, had errors up to 1.3 times these.)
+// P, U and M are carried negated (mP, mU, mM: pair instructions have no operand
+// negation, and the roundings are the same either way): 18.9 -> 18.2 ms for 100
+// iterations of the first workload below.
 // The nodes go in pairs (i, i+1) on the two lanes of pair instructions, the
 // sums kept per lane and folded at the end; ptxas may fuse a pair multiply
 // into the following pair add, and this is the model's only form, so every
@@ -691,8 +694,8 @@ GX_HD void nexi_node(int nx, float h, int i, float2& x2, float2& w, float2& wx2,
 // against 48 cycles of the SFU's 6 operations) with the adjoint, the SFU
 // without it (17 pair instructions).  Measured, 62 pair instructions with the
 // node positions recomputed in the loop -> this form: 328,050 voxels x 24
-// shells x 14 nodes, MSE, 229 -> 187 us an iteration; 100,003 voxels x 100
-// nodes, Rician loss, 514 -> 414 us; Goodman-Weare steps of 20,000 voxels x 64
+// shells x 14 nodes, MSE, 229 -> 179 us an iteration; 100,003 voxels x 100
+// nodes, Rician loss, 514 -> 403 us; Goodman-Weare steps of 20,000 voxels x 64
 // walkers 435 -> 344 us (SFU 82 % active).  The table is read from shared
 // memory: through the constant bank the same kernels take 2-20 % longer.
 // Nodes beyond kNodeTab are computed in the loop.
@@ -711,9 +714,9 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
     int nx = P.nx;
     float h = P.h;
     int nsh = P.n_shell;
-    const float2 z2 = make_float2(0.f, 0.f), one = bcast2(1.0f), two = bcast2(2.0f), mtwo = bcast2(-2.0f);
-    const float2 mhalf = bcast2(-0.5f), mexp = bcast2(-0.5f * kLog2e);  // exp(-L/2) = 2^(-L log2(e)/2)
-    const float2 f2 = bcast2(f), f2x2 = bcast2(2.0f * f), omf2x2 = bcast2(2.0f * omf);
+    const float2 z2 = make_float2(0.f, 0.f), one = bcast2(1.0f), mone = bcast2(-1.0f), two = bcast2(2.0f), mtwo = bcast2(-2.0f);
+    const float2 half = bcast2(0.5f), mexp = bcast2(-0.5f * kLog2e);  // exp(-L/2) = 2^(-L log2(e)/2)
+    const float2 mf2 = bcast2(-f), f2x2 = bcast2(2.0f * f), omf2x2 = bcast2(2.0f * omf);
     for (int j = 0; j < nsh; ++j) {
         float b = P.bval[j], D = P.delta[j];
         float d2 = b * De;
@@ -724,7 +727,7 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
         float q4 = 4.0f * r1 * r2;
         float bDa = b * Da;
         float fd2 = omf * d2;
-        const float2 bDa2 = bcast2(bDa), base2 = bcast2(base), q42 = bcast2(q4), c12 = bcast2(c1), fd22 = bcast2(fd2);
+        const float2 bDa2 = bcast2(bDa), base2 = bcast2(base), q42 = bcast2(q4), c12 = bcast2(c1), mfd22 = bcast2(-fd2);
         const float2 bDax2 = bcast2(2.0f * bDa), md2x2 = bcast2(-2.0f * d2), r1x2 = bcast2(2.0f * r1), r2x2 = bcast2(2.0f * r2);
         float2 S0p = z2, Sfp = z2, Sd1p = z2, Sd2p = z2, Sr1p = z2, Sr2p = z2;
         float2 S0q = z2, Sfq = z2, Sd1q = z2, Sd2q = z2, Sr1q = z2, Sr2q = z2;  // weighted with p2 (lmax 2)
@@ -749,31 +752,29 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
             const float2 R = make_float2(fminf(rs.x, 0.5f / EPS), fminf(rs.y, 0.5f / EPS));
             const float2 L1 = add2(c12, d1);
             const float2 LM = sub2(L1, L2), LP = add2(L1, L2);
-            const float2 N = fma2(mhalf, LM, fma2(f2, d1, fd22));
-            const float2 Pp = mul2(N, R);
+            const float2 mP = mul2(fma2(half, LM, fma2(mf2, d1, mfd22)), R);
             const float2 xm = mul2(LM, mexp), xp = mul2(LP, mexp);
             const float2 em = make_float2(ex2_ftz(xm.x), ex2_ftz(xm.y));
             const float2 ep = make_float2(ex2_ftz(xp.x), ex2_ftz(xp.y));
-            const float2 omP = sub2(one, Pp);
-            const float2 U = mul2(omP, em);
-            const float2 M = fma2(Pp, ep, U);
+            const float2 mU = mul2(sub2(mone, mP), em);
+            const float2 mM = fma2(mP, ep, mU);
             const float2 Nb = mul2(sub2(ep, em), R);
-            const float2 Wr = mul2(fma2(Nb, fma2(mtwo, Pp, one), fma2(two, U, make_float2(-M.x, -M.y))), R);
+            const float2 Wr = mul2(fma2(Nb, fma2(two, mP, one), fma2(mtwo, mU, mM)), R);
             const float2 W = make_float2(rs.x < 0.5f / EPS ? Wr.x : 0.0f, rs.y < 0.5f / EPS ? Wr.y : 0.0f);
-            const float2 av = add2(M, Nb), ma = make_float2(-av.x, -av.y);
+            const float2 ma = sub2(mM, Nb);
             const float2 dd = fma2(bDax2, x2, md2x2);            // 2 (d1 - d2)
             const float2 fb = mul2(Nb, dd);                      // each derivative times two
             const float2 gp = fma2(s, W, ma), gm = fma2(make_float2(-s.x, -s.y), W, ma);
             const float2 d1b = fma2(f2x2, Nb, gp), d2b = fma2(omf2x2, Nb, gm);
             const float2 r1b = fma2(r2x2, W, gp), r2b = fma2(r1x2, W, gm);
-            S0p = fma2(wt, M, S0p);
+            S0p = fma2(wt, mM, S0p);
             Sfp = fma2(wt, fb, Sfp);
             Sd1p = fma2(wx2, d1b, Sd1p);
             Sd2p = fma2(wt, d2b, Sd2p);
             Sr1p = fma2(wt, r1b, Sr1p);
             Sr2p = fma2(wt, r2b, Sr2p);
             if (LMAX2) {
-                S0q = fma2(wp2, M, S0q);
+                S0q = fma2(wp2, mM, S0q);
                 Sfq = fma2(wp2, fb, Sfq);
                 Sd1q = fma2(mul2(wp2, x2), d1b, Sd1q);
                 Sd2q = fma2(wp2, d2b, Sd2q);
@@ -792,7 +793,7 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
             g[3] = hh * ((Sr1.x + Sr1.y) + r2s * rf) * D;
         };
         {
-            const float S0 = S0p.x + S0p.y;
+            const float S0 = -(S0p.x + S0p.y);
             float S = S0 * h;
             float g[4], dS[NP];
             partials(Sfp, Sd1p, Sd2p, Sr1p, Sr2p, g);
@@ -814,7 +815,7 @@ __device__ __forceinline__ void nexi_shells(const DevProtocol& P, const float* t
         }
         if (LMAX2) {
             const float p2 = th[NP - 1];
-            const float T0 = S0q.x + S0q.y;
+            const float T0 = -(S0q.x + S0q.y);
             const float T = T0 * h;
             const float sg = p2 * (float)((T > 0.0f) - (T < 0.0f));
             float S = p2 * fabsf(T);

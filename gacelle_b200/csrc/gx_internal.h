@@ -52,6 +52,7 @@ struct AdamParams {
     float* ckpt;                  // checkpoint slots, each 3*np*nvtot floats
     int ckpt_every;
     float* res_out;               // [nm][nvtot] or nullptr
+    int* wait_err;                // set by a fused kernel whose wait ran out; nullptr: kernels without waits only
     // TV
     int n_reg;
     int reg_param[kMaxReg];
@@ -78,6 +79,10 @@ cudaError_t launch_init_state(const AdamParams& a, const float* theta0, double r
 cudaError_t launch_fused(const AdamParams& a, int model, int loss, bool stats, int e_begin,
                          int e_end, int update_last, bool record, int block, int nblocks,
                          cudaStream_t s);
+// Multiprocessors of the current device; whether a NEXI fit of nvtot padded
+// voxels may take the kernel whose waits need AdamParams::wait_err.
+int sm_count();
+bool nexi_turns(int nvtot, int nsm);
 // Largest launch block (multiple of 32) the fused kernel variant of this job
 // accepts: its thread limit and its per-block shared memory; 0 on error.
 int fused_block_limit(const AdamParams& a, int model, int loss, bool stats);

@@ -234,6 +234,32 @@ def test_history_groups(ctx, iters, block):
         assert np.all(np.isfinite(a["loss_history"]))
 
 
+@pytest.mark.parametrize("n,iters,over", [
+    (99_400, 3, {}), (99_500, 2, {}), (100_003, 59, {"tol": 1e-30}),
+    (123_457, 7, {"convergenceStepTol": 1e-30, "convergenceGradTol": 1e-30, "lossFunction": "l2"}),
+])
+def test_nexi_turns(ctx, n, iters, over):
+    """Voxels that fill an SM's warps more than once are fitted in turns of
+    (32 voxels, some epochs); with one epoch a launch (chunk) the general kernel
+    fits them.  Same parameters bit for bit, around the voxel count of the rule,
+    with a last turn of fewer epochs, with weights and statistics; the history's
+    FP64 sums of equal terms (about 4000) in another order: 4000 x 2^-53."""
+    from helpers import run_engine
+    rng = np.random.default_rng(n)
+    _, om = models("nexi")
+    th = random_theta("nexi", n, rng)
+    y = oracle.forward(om, th) + 0.01 * rng.standard_normal((24, n))
+    w = rng.uniform(0.3, 1.0, y.shape).astype(np.float32) if "lossFunction" in over else None
+    th0 = np.tile(np.array([[0.4], [2.0], [1.0], [0.05]], np.float32), (1, n))
+    opts = dict({"tol": 1e-30}, **over)
+    a, b = (run_engine("nexi", y, th0, fitting(iteration=iters, chunk=c, **opts), NAMES["nexi"], context=ctx, weights=w)
+            for c in (0, 1))
+    for k in ("final_theta", "min_theta", "final_residual", "min_residual"):
+        assert np.array_equal(a[k], b[k]), k
+    assert a["min_niteration"] == b["min_niteration"]
+    assert np.allclose(a["loss_history"], b["loss_history"], rtol=1e-12, atol=0.0, equal_nan=True)
+
+
 @pytest.mark.parametrize("n", [75_700, 75_800])
 def test_r2s_pairs_rule(ctx, n):
     """Around the voxel count from which R2* takes two voxels a thread."""
