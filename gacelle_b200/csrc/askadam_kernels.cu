@@ -869,6 +869,7 @@ struct DsigAcc {
     int s;
     float g[NP];
     __device__ __forceinline__ void add(int m, float S, const float (&dS)[NP]) {
+        if (MayBeNonFinite<NP>::value && !isfinite(S)) return;  // as LossAcc does
         float d = ds[m * s];
 #pragma unroll
         for (int k = 0; k < NP; ++k) g[k] += d * dS[k];
@@ -1020,6 +1021,49 @@ __global__ void plain_update_kernel(AdamParams a, PlainBufs b, int e) {
     }
 }
 
+// LossAcc for parameters from outside the bounds (gradient_kernel): every
+// prediction is tested, as plain_loss_kernel does.  A non-finite one counts as
+// 0 with the derivative 0; for R2* and R1-R2* that 0 multiplies the model's
+// derivatives, as in plain_adjoint_kernel (0 x infinity leaves NaN in that voxel's
+// gradient).  FUSED: the fused MSE sums, which have no test: the sum of squares
+// of a voxel with a non-finite prediction is not finite either, and the caller
+// then evaluates it again without FUSED.  Strides are 64-bit: arrays may hold more than 2^31 values.
+template <int LOSS, int NP, bool FUSED>
+struct GradAcc {
+    static constexpr bool kMse = FUSED && LOSS == kMSE;
+    float total;
+    float g[NP];
+    const float* y;   // measurement m at y[m*n], and so on
+    const float* w;   // nullptr: unit weights
+    float* res;       // nullptr or residual output
+    size_t n, rs;     // rs = n (the models' name of the residual stride)
+    LossAux aux;
+    float mse_scale, hd;
+
+    __device__ __forceinline__ void add(int m, float S, const float (&dS)[NP]) {
+        const bool bad = !isfinite(S);
+        const float s = bad ? 0.0f : S;
+        float d;
+        if constexpr (LOSS == kMSE) {
+            d = s - y[m * n];
+            total = __fmaf_rn(d, d, total);
+            if (res) res[m * n] = mse_scale * d * d;
+        } else {
+            const float l = loss_elem<LOSS>(s, y[m * n], w ? w[m * n] : 1.0f, aux, mse_scale, hd, d);
+            total += l;
+            if (res) res[m * n] = l;
+        }
+        if (MayBeNonFinite<NP>::value && bad) return;
+        if (bad) d = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NP; ++k) g[k] = __fmaf_rn(d, dS[k], g[k]);
+    }
+    __device__ __forceinline__ void finish() {
+        if constexpr (LOSS == kMSE) mse_finish(total, g, mse_scale);
+    }
+    __device__ __forceinline__ float meas(int m) const { return y[m * n]; }
+};
+
 // One evaluation of loss and d loss / d theta (askadam.model_gradient without a
 // regulariser) on the caller's arrays [.][nvox]: model, loss and adjoint in one
 // pass, so that the measurements and parameters are read once and gradient and
@@ -1052,17 +1096,28 @@ __global__ void gradient_kernel(AdamParams a, const float* theta, float* gtheta,
         float th[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) th[k] = theta[(size_t)k * a.nvtot + v];
-        LossAcc<LOSS, NP> acc;
-        acc.total = 0.0f;
+        auto eval = [&](auto& acc) {
+            acc.total = 0.0f;
 #pragma unroll
-        for (int k = 0; k < NP; ++k) acc.g[k] = 0.0f;
-        acc.y = a.data + v; acc.ys = a.nvtot;
-        acc.w = a.weights ? a.weights + v : nullptr; acc.ws = a.nvtot;
-        acc.aux = make_loss_aux(voxel_sigma(a, v));
-        acc.mse_scale = a.mse_scale; acc.hd = a.huber_delta;
-        acc.res = a.res_out ? a.res_out + v : nullptr;
-        acc.rs = a.nvtot;
-        model_eval<MODEL>(s_P, th, va, acc);
+            for (int k = 0; k < NP; ++k) acc.g[k] = 0.0f;
+            acc.y = a.data + v;
+            acc.w = a.weights ? a.weights + v : nullptr;
+            acc.res = a.res_out ? a.res_out + v : nullptr;
+            acc.n = acc.rs = (size_t)a.nvtot;
+            acc.aux = make_loss_aux(voxel_sigma(a, v));
+            acc.mse_scale = a.mse_scale; acc.hd = a.huber_delta;
+            model_eval<MODEL>(s_P, th, va, acc);
+        };
+        GradAcc<LOSS, NP, true> acc;
+        eval(acc);
+        if constexpr (LOSS == kMSE && !MayBeNonFinite<NP>::value)
+            if (!isfinite(acc.total)) {
+                GradAcc<LOSS, NP, false> tested;
+                eval(tested);
+                acc.total = tested.total;
+#pragma unroll
+                for (int k = 0; k < NP; ++k) acc.g[k] = tested.g[k];
+            }
         acc.finish();
         loss = acc.total;
         if (gtheta)

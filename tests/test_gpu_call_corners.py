@@ -1,0 +1,88 @@
+"""Corners of the calls' ranges: values, sizes and options at which a kernel's
+shortcut, index or wait could go wrong, each against the oracle, the general
+form of the same kernel or a plain restatement."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from gacelle_b200 import _lib
+from gacelle_b200 import askadam_solver as gx_askadam
+
+from helpers import NAMES, bounds, fitting, models, random_theta
+
+pytestmark = pytest.mark.gpu
+
+
+def _gradient(ctx, kind, y, th, b1=None, **over):
+    """gx_model_gradient on host arrays: fidelity, gradient, residual."""
+    n = th.shape[1]
+    gxm, _ = models(kind)
+    lb, ub = bounds(kind)
+    opts = gx_askadam.build_opts(fitting(**over), NAMES[kind], lb, ub)
+    vol = _lib.GxVolume()
+    vol.dims[0], vol.dims[1], vol.dims[2], vol.nvox = n, 1, 1, n
+    g, r, fid = np.zeros_like(th), np.zeros_like(y), C.c_double()
+    idx = np.arange(n, dtype=np.int32)
+    vol.data, vol.grid_index = y.ctypes.data_as(_lib._fp), idx.ctypes.data_as(_lib._i32p)
+    if b1 is not None:
+        vol.b1 = b1.ctypes.data_as(_lib._fp)
+    _lib.check(_lib.lib().gx_model_gradient(ctx.ptr, C.byref(gxm.s), _lib.MEM_HOST, C.byref(vol), C.byref(opts),
+                                            th.ctypes.data, g.ctypes.data, r.ctypes.data, None, C.byref(fid), None))
+    return fid.value, g, r
+
+
+@pytest.mark.parametrize("loss", ["mse", "l2"])
+@pytest.mark.parametrize("kind", ["r2s", "r1r2s", "nexi"])
+def test_gradient_of_non_finite_predictions(ctx, kind, loss):
+    """Voxels whose parameters (or B1) are not numbers, or make the signal
+    overflow at every or at some echo times: their non-finite predictions count
+    as 0 (utils.set_nan_inf_zero, utils/askadam.m:80), so that the call's loss
+    stays a number, as the oracle's does.  With and without a regulariser, whose
+    paths are different kernels, the fidelity, the residuals and the gradient of
+    an unregularised parameter are the same (bars of the gradient parity tests)."""
+    rng = np.random.default_rng(3)
+    n = 150
+    _, om = models(kind)
+    lb, ub = bounds(kind)
+    th = random_theta(kind, n, rng).astype(np.float32)
+    y = (oracle.forward(om, th.astype(np.float64)) + 0.02 * rng.standard_normal((24 if kind != "r2s" else 12, n))).astype(np.float32)
+    b1 = rng.uniform(0.8, 1.2, n).astype(np.float32) if kind == "r1r2s" else None
+    odd = [5, 77, 149]
+    th[0, 5], th[1, 77] = np.nan, np.nan
+    if kind == "nexi":
+        th[3, 149] = np.inf
+    else:
+        th[-1, 149] = -1e6      # overflows at every echo time, in 64 bits as well
+        th[-1, 20] = np.inf     # a signal of 0, finite
+        odd.append(100)
+        th[-1, 100] = -1e5      # in 32 bits at every echo time, in 64 bits at the later ones: not compared below
+        y[:, 100] = 0.0
+    if b1 is not None:
+        b1[64] = np.nan
+        odd.append(64)
+    fid, g, r = _gradient(ctx, kind, y, th, b1, lossFunction=loss)
+    assert np.isfinite(fid)
+    # the oracle, over the voxels whose predictions are the same numbers in 32 and 64 bits (its NEXI
+    # forward's fmin makes a NaN 1), at the same mean
+    keep = np.setdiff1d(np.arange(n), odd if kind == "nexi" else [100])
+    f = fitting(lossFunction=loss)
+    vol = oracle.Volume(y[:, keep].astype(np.float64), b1=None if b1 is None else b1[keep].astype(np.float64),
+                        norm_nvox=float(n))
+    Lo, go, ro, _, _ = oracle.model_gradient(om, vol, oracle.adam_opts(lb, ub, f), th[:, keep].astype(np.float64))
+    if kind != "nexi":
+        assert np.isfinite(Lo) and abs(fid - Lo) <= 1e-5 * abs(Lo) + 1e-7
+    assert np.all(np.abs(r[:, keep] - ro) <= 2e-4 * np.abs(ro) + 2e-5)
+    fine = np.setdiff1d(np.arange(n), odd)
+    at = np.searchsorted(keep, fine)
+    for k in range(th.shape[0]):
+        assert np.max(np.abs(g[k][fine] - go[k][at])) <= 1e-3 * np.max(np.abs(go[k][at])) + 1e-12
+    # the op-by-op kernels, which a regulariser of the last parameter takes
+    fid2, g2, r2 = _gradient(ctx, kind, y, th, b1, lossFunction=loss, regmap=[NAMES[kind][-1]], TVmode="2D",
+                             **{"lambda": [1e-6]})
+    assert abs(fid - fid2) <= 1e-5 * abs(fid2)
+    np.testing.assert_allclose(r, r2, rtol=2e-5, atol=2e-6)
+    assert np.array_equal(np.isnan(g[:-1]), np.isnan(g2[:-1]))
+    for k in range(th.shape[0] - 1):
+        assert np.nanmax(np.abs(g[k] - g2[k])) <= 1e-3 * np.nanmax(np.abs(g2[k])) + 1e-12
