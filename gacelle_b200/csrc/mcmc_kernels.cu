@@ -69,6 +69,12 @@ __global__ void gw_partner_kernel(McmcParams p, int* partner, int nsteps, int gl
     else rb_anchors_dev(p.seed, k, (global_block ? kTagGwGRbPart : kTagGwRbPart) | bits, p.nwalker, out);
 }
 
+// Residual of one R2* echo, M0 exp(-te R2*) - y, with its roundings stated: the
+// log-likelihood and the screen below form it alike, whatever the compiler fuses.
+__device__ __forceinline__ float r2s_residual(float te_l2e, float M0, float R2, float y) {
+    return fma1(M0, ex2_ftz(mul1(-te_l2e, R2)), -y);
+}
+
 // logP_Gaussian (utils/logP_Gaussian.m:18-20) of the model's parameters and
 // the noise sigma (the last of the NV variables, a compile-time index so that
 // the caller's parameter vector stays in registers); y / w with strides.
@@ -77,11 +83,20 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
                                              int ys, const float* w, int ws, const VoxAux& va) {
     constexpr int NP = ModelNP<MODEL>::value;
     static_assert(NV == NP + 1, "the variables are the model's parameters and the noise sigma");
-    SosSink<NP> sink{y, ys, w, ws, 0.0};
-    model_eval<MODEL>(P, x, va, sink);
+    double sos = 0.0;
+    if constexpr (MODEL == kR2S) {
+        for (int m = 0; m < nm; ++m) {
+            const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m * ys]);
+            sos += (double)mul1(mul1(w ? w[m * ws] : 1.0f, r), r);
+        }
+    } else {
+        SosSink<NP> sink{y, ys, w, ws, 0.0};
+        model_eval<MODEL>(P, x, va, sink);
+        sos = sink.sos;
+    }
     const double noise = (double)x[NV - 1];
     const double n2 = noise * noise;
-    return -sink.sos / (2.0 * n2) - 0.5 * nm * log(6.283185307179586 * n2);
+    return -sos / (2.0 * n2) - 0.5 * nm * log(6.283185307179586 * n2);
 }
 
 // Screened acceptance (R2*, unit weights, up to kScreenM measurements).
@@ -94,7 +109,7 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
 // proposal in 10^4; so every decision is the FP64 one.  With n the noise,
 // a = sos / (2 n^2) and the constant nm log(2 pi) / 2 cancelling,
 //   log p' - log p = (a - a') + nm (log n - log n').
-// Error, with e = 2^-24: the residuals are the FP64 form's (same operations);
+// Error, with e = 2^-24: the residuals are the FP64 form's (r2s_residual);
 // the FP32 sum of their nm squares and the FP64 sum of the rounded squares
 // differ by at most (nm + 1) e relative, a by at most another 6 e (n^2,
 // reciprocal of 1 ulp, two products): (nm + 20) e.  __logf is within
@@ -112,11 +127,6 @@ constexpr int kScreenM = 16;
 struct Screen {
     float a, ln;  // sos / (2 n^2), log n
 };
-
-// Residual of one echo, M0 exp(-te R2*) - y, as log_prob_t forms it.
-__device__ __forceinline__ float r2s_residual(float te_l2e, float M0, float R2, float y) {
-    return fma1(M0, ex2_ftz(mul1(-te_l2e, R2)), -y);
-}
 
 // P: the protocol in the constant bank (compile-time indices); up to MAXM
 // echoes, without a test when the protocol fills the bound.

@@ -86,3 +86,47 @@ def test_gradient_of_non_finite_predictions(ctx, kind, loss):
     assert np.array_equal(np.isnan(g[:-1]), np.isnan(g2[:-1]))
     for k in range(th.shape[0] - 1):
         assert np.nanmax(np.abs(g[k] - g2[k])) <= 1e-3 * np.nanmax(np.abs(g2[k])) + 1e-12
+
+
+def _chain(ctx, te, y, x0, update, W, steps, lb, ub, step, weights=None, **over):
+    from gacelle_b200 import mcmc_solver
+    from gacelle_b200.models import gpuR2starMapping
+    m = gpuR2starMapping(te)
+    f = mcmc_solver.check_set_default_basic(dict({
+        "algorithm": "MH" if update == "mh" else "GW", "iteration": steps, "thinning": 3, "burnin": 0.0, "Nwalker": W,
+        "Ensembleupdate": "redblack" if update == "redblack" else "simultaneous", "lb": lb, "ub": ub,
+        "xStepSize": step, "seed": 21}, **over))
+    solver = mcmc_solver.mcmc(ctx)
+    return dict(solver._run(m, y, weights, x0, None, m.modelParams, f, True), n_accepted=solver.last_stats["n_accepted"])
+
+
+def _same_chains(ctx, n_te, update, noise, scale, nv, steps, blocks):
+    """Chains with the FP32 screen and, with unit weights as an array, those
+    decided in FP64 throughout, from the same starts."""
+    rng = np.random.default_rng(n_te)
+    te = np.linspace(2e-3, 40e-3, n_te)
+    th = np.vstack([scale * rng.uniform(0.5, 1.5, nv), rng.uniform(10, 60, nv)])
+    y = (th[0] * np.exp(-te[:, None] * th[1]) + noise * rng.standard_normal((n_te, nv))).astype(np.float32)
+    x0 = np.vstack([th, np.full(nv, noise)]).astype(np.float32)
+    lb, ub = [0.0, 0.1, 0.8 * noise], [2.0 * scale, 200.0, 4.0 * noise]
+    step = [noise, 50.0 * noise / scale, 0.2 * noise]  # of the posterior's width: about half of the moves are taken
+    ones = np.ones_like(y)
+    W = 1 if update == "mh" else 17
+    a, *rest = [_chain(ctx, te, y, x0, update, W, steps, lb, ub, step, w, blockSize=b)
+                for w, b in [(ones, blocks[0])] + [(None, b) for b in blocks]]
+    moved = np.mean(np.diff(a["posterior"][0].reshape(-1, nv), axis=0) != 0)
+    assert 0.05 < moved
+    for b in rest:
+        for key in ("posterior", "mean", "std"):
+            assert np.array_equal(a[key], b[key], equal_nan=True), key
+        assert a["n_accepted"] == b["n_accepted"]
+
+
+@pytest.mark.parametrize("noise", [0.02, 0.001])
+@pytest.mark.parametrize("n_te", [3, 8, 12, 16])
+@pytest.mark.parametrize("update,steps", [("simultaneous", 1500), ("redblack", 1500), ("mh", 6000)])
+def test_screened_decisions_are_the_fp64_ones(ctx, update, steps, n_te, noise):
+    """The screened acceptance takes every decision as the FP64 log-likelihoods
+    do, also at small noise, where a residual's last bit is worth most: whole
+    chains are equal bit for bit (both Metropolis-Hastings kernels)."""
+    _same_chains(ctx, n_te, update, noise, 1.0, 40, steps, (0, 64) if update == "mh" else (0,))
