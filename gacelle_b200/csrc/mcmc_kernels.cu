@@ -116,13 +116,18 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
 // 2^-21.4 absolute or 3 ulp relative of the logarithm, and the roundings of
 // the sums are below 2^-21 of their terms: 2^-20 of every term's magnitude
 // plus 2^-20 for every logarithm.  NaN and infinities fail both tests and go
-// to the FP64 form.  Measurements in registers, echo constants in the constant
-// bank; kernels for up to 8, 12 and 16 echoes, since a test per echo and one
-// chain of sums cost a tenth of the kernel.  12,013 voxels x 50 walkers x 500
+// to the FP64 form.  The noise's bounds have to keep 2 n^2 and its reciprocal
+// in FP32's normal range (kScreenMaxNoise), and n large enough that the squares
+// below 2^-126, which FP32 flushes, do not count: nm 2^-126 / (2 n^2) is at most
+// nm 2^-20 from 1e-16 on (kScreenMinNoise).
+// Measurements in registers, echo constants in the constant bank; kernels for
+// up to 8, 12 and 16 echoes, since a test per echo and one chain of sums cost a
+// tenth of the kernel.  12,013 voxels x 50 walkers x 500
 // steps, 12 echoes: 6.93 (all FP64) -> 3.65 ms; Metropolis-Hastings, 4096
 // voxels x 10,000 steps: 15.4 -> 6.1 ms (one dependent chain a voxel, 1.4-2.1
 // -> 0.6 us a step).
 constexpr int kScreenM = 16;
+constexpr float kScreenMinNoise = 1e-16f, kScreenMaxNoise = 1e18f;
 
 struct Screen {
     float a, ln;  // sos / (2 n^2), log n
@@ -1038,9 +1043,13 @@ static void gw_shape(const McmcParams& p, int block_hint, int* vpb, int* block, 
             sizeof(float) * ((size_t)(*vpb) * W * p.nvar + 2 * (size_t)(*vpb) * p.nm);
 }
 
-// The screen's bound holds for a sum of squares (no weights), and its
-// measurements are held in registers.
-static bool screened(const McmcParams& p) { return p.weights == nullptr && p.nm <= kScreenM; }
+// The screen's bound holds for a sum of squares (no weights) and for noises
+// (clamped to their bounds in every state) in its range; its measurements are
+// held in registers.
+static bool screened(const McmcParams& p) {
+    return p.weights == nullptr && p.nm <= kScreenM && p.lb[p.nvar - 1] >= kScreenMinNoise &&
+           p.ub[p.nvar - 1] <= kScreenMaxNoise;
+}
 
 bool mcmc_batched(const McmcParams& p, int model) {
     return p.algorithm == 0 && model == kR2S && screened(p) && p.nvox <= kMhBatchVoxels;

@@ -130,3 +130,11 @@ def test_screened_decisions_are_the_fp64_ones(ctx, update, steps, n_te, noise):
     do, also at small noise, where a residual's last bit is worth most: whole
     chains are equal bit for bit (both Metropolis-Hastings kernels)."""
     _same_chains(ctx, n_te, update, noise, 1.0, 40, steps, (0, 64) if update == "mh" else (0,))
+
+
+@pytest.mark.parametrize("scale,noise", [(1e-18, 1e-19), (1e-15, 1.5e-16), (1e-15, 1e-16), (1e6, 1e4), (1e19, 1e18)])
+@pytest.mark.parametrize("update,steps", [("simultaneous", 300), ("mh", 1200)])
+def test_screened_decisions_in_any_unit(ctx, update, steps, scale, noise):
+    """The same for data in units whose noise (or its square) leaves FP32's
+    normal range, where the screen's bound does not hold."""
+    _same_chains(ctx, 12, update, noise, scale, 40, steps, (0, 64) if update == "mh" else (0,))
