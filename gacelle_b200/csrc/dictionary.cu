@@ -121,7 +121,9 @@ dict_match_kernel(const float* signals, int nvox, const float* dict, int ndict, 
     // list: the voxels that the tensor-core kernel left (count in stat)
     const int n = list ? min(stat->n_left, nvox) : nvox;
     if (list && n <= kFewLeft) return;  // dict_scan_kernel's
-    for (int i0 = blockIdx.x * kTile; i0 < n; i0 += gridDim.x * kTile) {
+    // 64-bit: with a grid over all voxels the step passes 2^31 from 2^30 voxels on
+    for (long long at = (long long)blockIdx.x * kTile; at < n; at += (long long)gridDim.x * kTile) {
+    const int i0 = (int)at;
     __syncthreads();  // the previous voxels' tile is consumed
     for (int q = tid; q < nm * kTile; q += kThreads) {
         int m = q / kTile, v = q % kTile;
@@ -687,7 +689,7 @@ cudaError_t launch_dictionary_match(const float* signals, int nvox, const float*
         auto kt = kernels[chunks_of(nm) - 2];
         e = cudaFuncSetAttribute(kt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kt<<<(nvox + kRows - 1) / kRows, kTensorThreads, smem, s>>>(signals, nvox, dict, ndict, nm, invE, op, best,
+        kt<<<(nvox - 1) / kRows + 1, kTensorThreads, smem, s>>>(signals, nvox, dict, ndict, nm, invE, op, best,
                                                                     best_sse, list, stat);
         dict_scan_kernel<<<kFewLeft, kThreads, 0, s>>>(signals, nvox, dict, ndict, nm, invE, best, best_sse, list, stat);
         g_kernel_launches += 2;
@@ -701,7 +703,7 @@ cudaError_t launch_dictionary_match(const float* signals, int nvox, const float*
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     // after the tensor-core kernel: the voxels it left (none as a rule)
-    const int blocks = (nvox + kTile - 1) / kTile;
+    const int blocks = (nvox - 1) / kTile + 1;
     k<<<tensor ? std::min(blocks, 4 * 148) : blocks, kThreads, smem, s>>>(signals, nvox, dict, ndict, nm, wt, invE, Cj, best,
                                                           best_sse, tensor ? list : nullptr, stat);
     ++g_kernel_launches;

@@ -138,3 +138,21 @@ def test_screened_decisions_in_any_unit(ctx, update, steps, scale, noise):
     """The same for data in units whose noise (or its square) leaves FP32's
     normal range, where the screen's bound does not hold."""
     _same_chains(ctx, 12, update, noise, scale, 40, steps, (0, 64) if update == "mh" else (0,))
+
+
+@pytest.mark.parametrize("weighted", [True, False])
+def test_dictionary_match_of_2_30_voxels(ctx, weighted):
+    """More than 2^30 voxels of one measurement against one entry, where 32-bit
+    steps over the work-list wrap: every voxel is matched, none twice wrongly."""
+    import torch
+    n = (1 << 30) + 65
+    y = torch.full((n,), 2.0, device="cuda")
+    y[-1] = 3.0
+    D, w = torch.tensor([0.5], device="cuda"), torch.tensor([1.5], device="cuda")
+    best = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().gx_dictionary_match(ctx.ptr, _lib.MEM_DEVICE, y.data_ptr(), n, D.data_ptr(), 1, 1,
+                                              w.data_ptr() if weighted else None, best.data_ptr(), None))
+    assert int(best.min()) == 0 and int(best.max()) == 0
+    del y, best
+    torch.cuda.empty_cache()
