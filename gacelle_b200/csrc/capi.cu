@@ -2026,7 +2026,7 @@ extern "C" gx_status gx_dictionary_match(gx_context* c, int32_t mem, const float
     unsigned char* op = nullptr;
     int* list = nullptr;
     DictStat* stat = nullptr;
-    if (dict_tensor_ok(ndict, nm, wt != nullptr)) {
+    if (dict_tensor_ok(nvox, ndict, nm, wt != nullptr)) {
         TRY(wsT(c, S_DICT_OP, dict_operand_bytes(ndict, nm), &op));
         TRY(wsT(c, S_DICT_LIST, (size_t)nvox, &list));
         TRY(wsT(c, S_DICT_STAT, 1, &stat));

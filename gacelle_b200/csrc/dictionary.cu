@@ -241,7 +241,7 @@ dict_match_kernel(const float* signals, int nvox, const float* dict, int ndict, 
 // 60 k clocks of a block's 240 k; two CTAs share an SM so that one works under
 // the other's waits.  500,000 voxels x 10^4 entries x 24 measurements: 14.6 ms
 // (FP64 pipe 47 %, operands from shared memory) -> 2.4 ms; 20,000 x 2000:
-// 0.12 ms; 1000 x 10^4: 0.18 ms.  The products are unrolled with descriptors
+// 0.11 ms; 1000 x 10^4: 0.17 ms.  The products are unrolled with descriptors
 // known at compile time: with descriptors loaded in a loop the issuing thread
 // took 126 clocks a product, unrolled it takes the pipe's 62.
 // ---------------------------------------------------------------------------
@@ -657,10 +657,24 @@ size_t dict_match_smem(int nm, bool weighted) {
 }
 
 // The tensor-core kernel takes unit weights, up to 64 measurements (three
-// operand tiles in shared memory) and dictionaries of at least one operand
-// tile (a smaller one is mostly padding) whose runs fit an item's 24 bits.
-bool dict_tensor_ok(int ndict, int nm, bool weighted) {
-    return !weighted && nm <= kMaxTensorNm && ndict >= kRows && ndict / kRun < (1 << 24);
+// operand tiles in shared memory) and dictionaries whose runs fit an item's 24
+// bits, from the number of entries on at which it wins over dict_match_kernel:
+// its launches, operand tiles and FP64 scores take 55-110 us whatever the
+// dictionary, which the other kernel's time is proportional to.  us, FP64 kernel /
+// tensor cores, 2000 voxels: 24 measurements, 600 entries 58 / 74, 1000: 79 /
+// 82, 2000: 132 / 95, 10,000: 547 / 171; 64 measurements, 1000: 133 / 132,
+// 2000: 235 / 146; 8 measurements, 1000: 53 / 70, 2000: 81 / 78, 5000: 169 /
+// 105.  60,000 voxels: 24 measurements, 300 entries 93 / 132, 600: 155 / 143; 8
+// measurements, 600: 87 / 110, 1000: 122 / 121; 48 measurements, 600: 253 / 269,
+// 1000: 388 / 294.
+// A dictionary so fine that most voxels overflow the kept runs (entries on a
+// curve of one parameter in random order, or all alike) pays for both kernels:
+// 200,000 voxels x 10,000 x 24, 6.1 / 6.9-7.2 ms, 2000 x 2000: 0.13 / 0.25; in
+// order of the parameter 6.1 / 1.2 ms.
+bool dict_tensor_ok(int nvox, int ndict, int nm, bool weighted) {
+    const bool many = nvox >= 40000;
+    const int least = nm < 16 ? (many ? 1024 : 1536) : (many && nm <= 32 ? 600 : 1024);
+    return !weighted && nm <= kMaxTensorNm && ndict >= least && ndict / kRun < (1 << 24);
 }
 
 size_t dict_operand_bytes(int ndict, int nm) { return (size_t)((ndict + kRows - 1) / kRows) * tile_bytes(nm); }

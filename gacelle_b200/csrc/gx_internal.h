@@ -179,7 +179,7 @@ struct DictStat {
     int pad;
 };
 size_t dict_match_smem(int nm, bool weighted);
-bool dict_tensor_ok(int ndict, int nm, bool weighted);
+bool dict_tensor_ok(int nvox, int ndict, int nm, bool weighted);
 size_t dict_operand_bytes(int ndict, int nm);
 cudaError_t launch_dictionary_match(const float* signals, int nvox, const float* dict, int ndict, int nm,
                                     const float* wt, double* invE, double* Cj, int* best, float* best_sse,

@@ -156,3 +156,61 @@ def test_dictionary_match_of_2_30_voxels(ctx, weighted):
     assert int(best.min()) == 0 and int(best.max()) == 0
     del y, best
     torch.cuda.empty_cache()
+
+
+def _match(ctx, y, D):
+    y, D = np.ascontiguousarray(y, np.float32), np.ascontiguousarray(D, np.float32)
+    best, sse = np.full(y.shape[1], -7, np.int32), np.full(y.shape[1], np.nan, np.float32)
+    _lib.check(_lib.lib().gx_dictionary_match(ctx.ptr, _lib.MEM_HOST, y.ctypes.data, y.shape[1], D.ctypes.data,
+                                              D.shape[1], y.shape[0], None, best.ctypes.data, sse.ctypes.data))
+    return best, sse, ctx.timing()["kernel_launches"]
+
+
+def _scores(y, D):
+    """sse [voxel, entry] in FP64 by the expanded form; NaN for an entry without a norm."""
+    y, D = np.asarray(y, np.float32).astype(np.float64), np.asarray(D, np.float32).astype(np.float64)
+    with np.errstate(divide="ignore", invalid="ignore", over="ignore"):
+        return (y * y).sum(0)[:, None] - (y.T @ D) ** 2 / (D * D).sum(0)
+
+
+@pytest.mark.parametrize("nm,nvox,entries,tensor", [
+    (1, 127, 1535, False), (1, 1, 1536, True), (8, 129, 1537, True), (15, 260, 1663, True), (16, 128, 1023, False),
+    (16, 1, 1024, True), (17, 127, 1025, True), (24, 129, 1151, True), (24, 260, 1152, True), (33, 257, 1153, True),
+    (48, 3, 1200, True), (56, 130, 1281, True), (64, 383, 1408, True), (65, 129, 1408, False),
+    (24, 40000, 599, False), (24, 40001, 600, True), (33, 40000, 1023, False), (8, 39999, 1100, False)])
+def test_dictionary_rule_and_tiles(ctx, nm, nvox, entries, tensor):
+    """Both kernels on either side of the rule (entries by measurements and
+    voxels) and around the 128-row operand tiles, at scales from 1e-20 to 1e20:
+    the entry of least FP64 score, or one whose score equals it to 1e-12 of the voxel's
+    energy.  The tensor-core path takes four launches, the FP64 kernel two."""
+    rng = np.random.default_rng(nm * 1000 + nvox)
+    y = rng.standard_normal((nm, nvox)) * 10.0 ** rng.uniform(-10, 10, nvox)
+    D = rng.standard_normal((nm, entries)) * 10.0 ** rng.uniform(-10, 10, entries)
+    best, sse, launches = _match(ctx, y, D)
+    assert launches == (4 if tensor else 2)
+    at = np.arange(nvox) if nvox < 1000 else rng.permutation(nvox)[:1000]
+    s = _scores(y[:, at], D)
+    A = (np.asarray(y[:, at], np.float32).astype(np.float64) ** 2).sum(0)
+    got = s[np.arange(at.size), best[at]]
+    assert np.all(got - s.min(1) <= 1e-12 * A)
+    assert np.all(np.abs(sse[at] - got) <= 1e-6 * np.abs(got) + 1e-12 * A)
+
+
+def test_dictionary_special_values_on_the_tensor_cores(ctx):
+    """Zero voxels take the first entry with a norm, voxels and entries that are
+    not numbers match nothing, and of equal entries the first wins, with a
+    dictionary that the tensor-core kernel takes."""
+    rng = np.random.default_rng(8)
+    D = np.abs(rng.standard_normal((20, 1700))) + 0.1
+    D[:, 0] = 0.0
+    D[3, 1], D[4, 2] = np.nan, np.inf
+    D[:, 300:400] = D[:, 200:300]
+    y = D[:, rng.integers(200, 1700, 150)] * 3.0 + 0.01 * rng.standard_normal((20, 150))
+    y[:, 0] = 0.0
+    y[5, 1], y[6, 2] = np.nan, np.inf
+    best, sse, launches = _match(ctx, y, D)
+    assert launches == 4
+    assert best[0] == 3 and sse[0] == 0.0
+    assert best[1] == best[2] == -1 and np.all(np.isinf(sse[1:3]))
+    assert np.array_equal(best[3:], np.nanargmin(_scores(y[:, 3:], D), axis=1))
+    assert not np.any((best >= 300) & (best < 400))
