@@ -1898,7 +1898,7 @@ extern "C" gx_status gx_mcmc(gx_context* c, const gx_model* model, int32_t mem, 
         if (partner) CK(launch_mcmc_partners(p, partner, c->stream));
         int block = o->block_size;
         if (block == 0 && ng == 0 && autotune_enabled() && !mcmc_batched(p, id)) TRY(tune_mcmc(c, p, id, &block, &tuned_now));
-        block_used = block > 0 ? block : 128;
+        block_used = o->algorithm == GX_MCMC_MH ? mcmc_mh_block(p, id, block) : (block > 0 ? block : 128);
         float* xstate;
         double* lpstate;
         TRY(wsT(c, S_MC_X, (size_t)nvar * nv * W, &xstate));

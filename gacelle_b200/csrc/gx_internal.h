@@ -232,6 +232,7 @@ cudaError_t launch_mcmc_partners(const McmcParams& p, int* partner, cudaStream_t
 // (= rows of the partial-sum table) and dynamic shared memory.
 void gwg_launch_shape(const McmcParams& p, int block_hint, int* vpb, int* block, int* nblocks, size_t* smem);
 int mcmc_steps_per_launch(const McmcParams& p);
+int mcmc_mh_block(const McmcParams& p, int model, int block_hint);  // threads per block of a Metropolis-Hastings launch
 bool mcmc_batched(const McmcParams& p, int model);  // the kernel with a block of its own (no shape to tune)
 // Node table of a NEXI protocol (capi.cu); its place in dynamic shared memory.
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;

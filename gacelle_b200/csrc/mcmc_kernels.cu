@@ -1055,6 +1055,39 @@ bool mcmc_batched(const McmcParams& p, int model) {
     return p.algorithm == 0 && model == kR2S && screened(p) && p.nvox <= kMhBatchVoxels;
 }
 
+template <int MODEL>
+static decltype(&mh_kernel<MODEL, ModelNP<MODEL>::value + 1, 0>) mh_kernel_fn(const McmcParams& p) {
+    constexpr int NV = ModelNP<MODEL>::value + 1;
+    if constexpr (MODEL == kR2S)
+        if (screened(p))
+            return p.nm <= 8 ? mh_kernel<MODEL, NV, 8> : p.nm <= 12 ? mh_kernel<MODEL, NV, 12> : mh_kernel<MODEL, NV, 16>;
+    return mh_kernel<MODEL, NV, 0>;
+}
+
+// Threads per block of a Metropolis-Hastings launch: the chosen block up to what the
+// kernel's registers leave (a chain does not depend on its block).
+template <class K>
+static cudaError_t mh_block_of(K kernel, int block_hint, int* block) {
+    *block = block_hint > 0 ? block_hint : 128;
+    if (*block <= 512 || *block > 1024) return cudaSuccess;  // always fits; refused by the launch
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess) *block = std::min(*block, fa.maxThreadsPerBlock / 32 * 32);
+    return e;
+}
+
+int mcmc_mh_block(const McmcParams& p, int model, int block_hint) {
+    int block = block_hint;
+    if (mcmc_batched(p, model) && block_hint <= 0) return 128;
+    switch (model) {
+    case kR2S: mh_block_of(mh_kernel_fn<kR2S>(p), block_hint, &block); break;
+    case kR1R2S: mh_block_of(mh_kernel_fn<kR1R2S>(p), block_hint, &block); break;
+    case kNEXI: mh_block_of(mh_kernel_fn<kNEXI>(p), block_hint, &block); break;
+    default: mh_block_of(mh_kernel_fn<kNEXI2>(p), block_hint, &block); break;
+    }
+    return block;
+}
+
 // Steps [k0, k1] of repetition rr as one launch (init: the walkers start at k0 == 1).
 template <int MODEL>
 static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k0, int k1, float* xstate,
@@ -1079,18 +1112,18 @@ static cudaError_t mcmc_launch_steps(McmcParams p, int block_hint, int rr, int k
         }
         k<<<nb, block, smem, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, lpstate, sum, sumsq);
     } else {
-        const int block = block_hint > 0 ? block_hint : 128;
-        const int nb = (p.nvox + block - 1) / block;
-        auto k = mh_kernel<MODEL, NV, 0>;
-        if constexpr (MODEL == kR2S) {
+        if constexpr (MODEL == kR2S)
             if (block_hint <= 0 && mcmc_batched(p, MODEL)) {
                 auto kb = p.nm <= 8 ? mh_batch_kernel<8> : p.nm <= 12 ? mh_batch_kernel<12> : mh_batch_kernel<16>;
                 kb<<<(p.nvox + 31) / 32, 128, 0, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, sum, sumsq);
                 ++g_kernel_launches;
                 return cudaGetLastError();
             }
-            if (screened(p)) k = p.nm <= 8 ? mh_kernel<MODEL, NV, 8> : p.nm <= 12 ? mh_kernel<MODEL, NV, 12> : mh_kernel<MODEL, NV, 16>;
-        }
+        auto k = mh_kernel_fn<MODEL>(p);
+        int block;
+        const cudaError_t e = mh_block_of(k, block_hint, &block);
+        if (e != cudaSuccess) return e;
+        const int nb = (p.nvox + block - 1) / block;
         k<<<nb, block, 0, s>>>(p, rr, k0, k1, k0 == 1 ? 1 : 0, xstate, lpstate, sum, sumsq);
     }
     ++g_kernel_launches;

@@ -214,3 +214,40 @@ def test_dictionary_special_values_on_the_tensor_cores(ctx):
     assert best[1] == best[2] == -1 and np.all(np.isinf(sse[1:3]))
     assert np.array_equal(best[3:], np.nanargmin(_scores(y[:, 3:], D), axis=1))
     assert not np.any((best >= 300) & (best < 400))
+
+
+@pytest.mark.parametrize("kind,blocks", [("r2s", (544, 800)), ("r1r2s", (704, 736)), ("nexi", (512,)), ("nexi2", (544, 672))])
+@pytest.mark.parametrize("n_te", [12, 17])
+def test_mh_large_blocks(ctx, kind, blocks, n_te):
+    """Metropolis-Hastings takes a chosen block beyond the threads that its
+    registers leave, in blocks as large as they do: chains equal those of
+    128-thread blocks bit for bit."""
+    from gacelle_b200 import mcmc_solver
+    from gacelle_b200.models import gpuJointR1R2starMapping, gpuNEXI, gpuR2starMapping
+    te = np.linspace(2e-3, 40e-3, n_te)
+    if kind == "r2s":
+        m = gpuR2starMapping(te)
+    elif kind == "r1r2s":
+        m = gpuJointR1R2starMapping(te, 0.03, [5.0, 20.0])
+    else:
+        m = gpuNEXI(np.tile([1.0, 2.5, 4.0, 6.0, 8.0, 10.0], 4), np.repeat([20.0, 27.0, 35.0, 49.0], 6))
+        m._gx_model = lambda: models(kind)[0]
+    rng = np.random.default_rng(6)
+    nv = 900
+    _, om = models(kind, **({"te": te} if kind[0] == "r" else {}))
+    th = random_theta(kind, nv, rng)
+    s = oracle.forward(om, th)
+    y = (s + 0.02 * rng.standard_normal(s.shape)).astype(np.float32)
+    x0 = np.vstack([th, np.full(nv, 0.02)]).astype(np.float32)
+    lb, ub = bounds(kind)
+    out = []
+    for block in (128,) + blocks:
+        f = mcmc_solver.check_set_default_basic({
+            "algorithm": "MH", "iteration": 40, "thinning": 2, "burnin": 0.0, "lb": list(lb) + [0.001],
+            "ub": list(ub) + [0.1], "xStepSize": [0.01] * (len(NAMES[kind]) + 1), "seed": 4, "blockSize": block})
+        solver = mcmc_solver.mcmc(ctx)
+        out.append(solver._run(m, y, None, x0, None, NAMES[kind] + ["noise"], f, True))
+        assert solver.last_timing["block_size"] <= block and solver.last_timing["block_size"] >= 128
+    for o in out[1:]:
+        for key in ("posterior", "mean", "std"):
+            assert np.array_equal(out[0][key], o[key], equal_nan=True), key
