@@ -295,9 +295,16 @@ __global__ void fused_kernel(AdamParams a, int e_begin, int e_end, int update_la
 // its echo loop unrolled, registers capped at 80 (unrolled and uncapped it
 // takes 128 and loses half of the resident warps).
 template <int LOSS, bool STATS>
-__global__ void __maxnreg__(80) fused_kernel_r1r2s(AdamParams a, int e_begin, int e_end, int update_last,
+__global__ void __maxnreg__(STATS && LOSS == kL2 ? 72 : 80) fused_kernel_r1r2s(AdamParams a, int e_begin, int e_end, int update_last,
                                                    int record) {
     fused_body<kR1R2S, LOSS, STATS>(a, e_begin, e_end, update_last, record);
+}
+
+// R2* with statistics under the other losses (MSE takes 56 registers and 1024 threads): capped at the 72
+// registers that a block of 896 threads leaves; uncapped 75.  The same line for R1-R2* under L2 above.
+template <int LOSS>
+__global__ void __maxnreg__(72) fused_kernel_r2s_stats(AdamParams a, int e_begin, int e_end, int update_last, int record) {
+    fused_body<kR2S, LOSS, true>(a, e_begin, e_end, update_last, record);
 }
 
 // NEXI with lmax 0: registers capped at 96 (20 warps an SM; uncapped up to
@@ -422,6 +429,7 @@ template <int MODEL, int LOSS, bool STATS>
 constexpr auto fused_kernel_fn() {
     if constexpr (MODEL == kNEXI) return &fused_kernel_nexi<MODEL, LOSS, STATS>;
     else if constexpr (MODEL == kR1R2S) return &fused_kernel_r1r2s<LOSS, STATS>;
+    else if constexpr (MODEL == kR2S && STATS && LOSS != kMSE) return &fused_kernel_r2s_stats<LOSS>;
     else return &fused_kernel<MODEL, LOSS, STATS>;
 }
 

@@ -251,3 +251,23 @@ def test_mh_large_blocks(ctx, kind, blocks, n_te):
     for o in out[1:]:
         for key in ("posterior", "mean", "std"):
             assert np.array_equal(out[0][key], o[key], equal_nan=True), key
+
+
+@pytest.mark.parametrize("kind,loss", [("r2s", "l1"), ("r2s", "l2"), ("r2s", "huber"), ("r2s", "gauss"),
+                                       ("r1r2s", "l2")])
+def test_fit_blocks_up_to_896(ctx, kind, loss):
+    """Fits with stopping statistics in blocks of 800 and 896 threads (72
+    registers a thread) equal those in blocks of 128, bit for bit."""
+    from helpers import run_engine
+    rng = np.random.default_rng(2)
+    n = 1000
+    _, om = models(kind)
+    s = oracle.forward(om, random_theta(kind, n, rng))
+    y = s + 0.01 * rng.standard_normal(s.shape)
+    th0 = np.tile(np.array([[1.0], [30.0]] if kind == "r2s" else [[1.0], [1.0], [30.0]], np.float32), (1, n))
+    a, *rest = (run_engine(kind, y, th0, fitting(iteration=12, blockSize=block, lossFunction=loss, noiseSigma=0.02,
+                                                 tol=-np.inf, convergenceStepTol=1e-30, convergenceGradTol=1e-30),
+                           NAMES[kind], context=ctx) for block in (128, 800, 896))
+    for b in rest:
+        for k in ("final_theta", "min_theta", "final_residual"):
+            assert np.array_equal(a[k], b[k]), k
