@@ -327,12 +327,15 @@ __global__ void __maxnreg__(96) fused_kernel_nexi(AdamParams a, int e_begin, int
 // round.  Between units a task's state lives in global memory; a unit waits for
 // the task's previous one (n units earlier, n > 20, of a warp of the same CTA:
 // the least unfinished unit never waits, so all end), with a limit on the wait.
+// A wait lasts a unit at most, and a unit's epochs are bounded by its nodes
+// (kRotNodes, some 35 ms at 0.13 us a node and shell with 20 warps an SM), so that
+// however long the fit the limit of 2 s only ends a wait that cannot end otherwise.
 // Per voxel the operations of fused_kernel_nexi.  24 warps at 80 registers: 0-2 %
 // slower or faster by size, and from 25 tasks on only.
 // ---------------------------------------------------------------------------
 constexpr int kRotWarps = 20;              // 640 threads x 96 registers
 constexpr int kRotTasks = 96;              // tasks of a CTA, at most
-constexpr long long kRotWait = 1LL << 32;  // clocks, about 2 s
+constexpr int kRotNodes = 1 << 18;         // epochs x shells x nodes of a unit, at most
 
 template <int LOSS, bool STATS>
 __global__ void __maxnreg__(96) fused_kernel_nexi_turns(AdamParams a, int e_begin, int e_end, int update_last, int record,
@@ -352,8 +355,9 @@ __global__ void __maxnreg__(96) fused_kernel_nexi_turns(AdamParams a, int e_begi
     stage_protocol(a.P, &s_P);
     stage_nodes(a.nodes, s_nodes);
     for (int i = tid; i < n; i += B) s_done[i] = 0;
-    if (tid == 0) s_err = 0;
+    if (tid == 0) s_err = *a.wait_err;  // an earlier launch's wait ran out: the call has failed
     __syncthreads();
+    if (s_err) return;
     const int nspan = (e_end - e_begin + span) / span;
     for (int u = warp; u < n * nspan; u += kRotWarps) {
         const int t = u % n, c = u / n;
@@ -361,9 +365,9 @@ __global__ void __maxnreg__(96) fused_kernel_nexi_turns(AdamParams a, int e_begi
             int bad = 0;
             if (lane == 0) {
                 const long long start = clock64();
-                while (s_done[t] < c && !bad) {
+                while (s_done[t] < c + a.wait_extra && !bad) {
                     __nanosleep(64);
-                    bad = s_err || clock64() - start > kRotWait;
+                    bad = s_err || clock64() - start > a.wait_limit;
                 }
                 if (bad) {
                     s_err = 1;
@@ -1201,14 +1205,15 @@ bool nexi_turns(int nvtot, int nsm) {
 }
 
 // Epochs of a unit of fused_kernel_nexi_turns (about 32 rounds a launch, for a
-// small last one), or 0: not for this launch.
+// small last one, and no more than kRotNodes allows), or 0: not for this launch.
 static int nexi_span(const AdamParams& a, int e_begin, int e_end, int nvox, int nsm, size_t* smem) {
     *smem = sizeof(NexiNodes) + sizeof(float) * (size_t)(32 * kRotWarps) * a.nm * (a.weights ? 2 : 1);
     const int epochs = e_end - e_begin + 1;
     if (!a.wait_err || nvox != a.nvtot || !nexi_turns(nvox, nsm) || epochs < 2 || a.P.nx > kNodeTab ||
         *smem + sizeof(DevProtocol) + 1024 > kMaxSmemPerBlock)
         return 0;
-    return std::max(1, (int)((long long)((nvox / 32 + nsm - 1) / nsm) * epochs / (32 * kRotWarps)));
+    const int rounds = (int)((long long)((nvox / 32 + nsm - 1) / nsm) * epochs / (32 * kRotWarps));
+    return std::max(1, std::min(rounds, kRotNodes / (a.P.nx * a.P.n_shell)));
 }
 
 template <int MODEL, int LOSS, bool STATS>

@@ -1151,6 +1151,8 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
     if (!J.tv && J.id == kNEXI && nexi_turns(J.nvtot, sm_count())) {
         TRY(wsT(c, S_WAIT_ERR, 1, &J.a.wait_err));
         CK(cudaMemsetAsync(J.a.wait_err, 0, sizeof(int), c->stream));
+        J.a.wait_limit = c->hooks.wait_limit_cycles > 0 ? c->hooks.wait_limit_cycles : kFusedWaitClocks;
+        J.a.wait_extra = c->hooks.barrier_extra_arrivals;
     }
     if (J.autotune) TRY(tune_fused(J));
     if (J.tv) {

@@ -53,6 +53,8 @@ struct AdamParams {
     int ckpt_every;
     float* res_out;               // [nm][nvtot] or nullptr
     int* wait_err;                // set by a fused kernel whose wait ran out; nullptr: kernels without waits only
+    long long wait_limit;         // clocks of such a wait, at most
+    int wait_extra;               // spans more than are made that it asks for (test hook)
     // TV
     int n_reg;
     int reg_param[kMaxReg];
@@ -79,6 +81,8 @@ cudaError_t launch_init_state(const AdamParams& a, const float* theta0, double r
 cudaError_t launch_fused(const AdamParams& a, int model, int loss, bool stats, int e_begin,
                          int e_end, int update_last, bool record, int block, int nblocks,
                          cudaStream_t s);
+// Bound of the waits in fused kernels, about 2 s: kRotNodes keeps what they wait for far below it.
+constexpr long long kFusedWaitClocks = 1LL << 32;
 // Multiprocessors of the current device; whether a NEXI fit of nvtot padded
 // voxels may take the kernel whose waits need AdamParams::wait_err.
 int sm_count();

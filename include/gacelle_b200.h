@@ -316,10 +316,12 @@ typedef struct {
      * an allocation failure would (GX_ENOMEM), without touching the device. */
     int32_t fail_alloc_at;
     /* > 0: bound, in SM clock cycles, of every wait in the persistent TV
-     * kernel (default about 2 s). */
+     * kernel and in the NEXI fit kernel whose warps take voxels in turns
+     * (default about 2 s). */
     int64_t wait_limit_cycles;
     /* > 0: the persistent kernel's grid barrier waits for this many arrivals
-     * more than the grid makes, so its bounded wait runs out: every CTA then
+     * more than the grid makes (the turns of the NEXI kernel for as many units
+     * more than are run), so its bounded wait runs out: every CTA then
      * returns and the call reports GX_ETIMEOUT, with the context usable. */
     int32_t barrier_extra_arrivals;
 } gx_test_hooks;

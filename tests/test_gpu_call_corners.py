@@ -271,3 +271,42 @@ def test_fit_blocks_up_to_896(ctx, kind, loss):
     for b in rest:
         for k in ("final_theta", "min_theta", "final_residual"):
             assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.fixture
+def own_ctx():
+    from gacelle_b200 import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _hooks(ctx, **kw):
+    h = _lib.GxTestHooks(0, kw.get("wait_limit_cycles", 0), kw.get("barrier_extra_arrivals", 0))
+    _lib.check(_lib.lib().gx_context_set_test_hooks(ctx.ptr, C.byref(h)))
+
+
+@pytest.mark.parametrize("chunk", [0, 8])
+def test_nexi_turns_wait_runs_out(own_ctx, chunk):
+    """A wait of the NEXI kernel that takes voxels in turns, for a unit that
+    nobody runs, ends at its limit: the call reports GX_ETIMEOUT (in one launch or several)
+    and the context stays usable."""
+    import time
+
+    from helpers import run_engine
+    rng = np.random.default_rng(1)
+    n = 100_003
+    _, om = models("nexi")
+    y = oracle.forward(om, random_theta("nexi", n, rng)) + 0.01 * rng.standard_normal((24, n))
+    th0 = np.tile(np.array([[0.4], [2.0], [1.0], [0.05]], np.float32), (1, n))
+    f = fitting(iteration=40, chunk=chunk, **({"tol": 1e-30} if chunk else {"tol": -np.inf}))
+    good = run_engine("nexi", y, th0, f, NAMES["nexi"], context=own_ctx)
+    _hooks(own_ctx, wait_limit_cycles=2_000_000, barrier_extra_arrivals=1000)
+    t0 = time.perf_counter()
+    with pytest.raises(_lib.GacelleError) as e:
+        run_engine("nexi", y, th0, f, NAMES["nexi"], context=own_ctx)
+    assert e.value.status == _lib.GX_ETIMEOUT
+    assert time.perf_counter() - t0 < 5.0
+    _hooks(own_ctx)
+    again = run_engine("nexi", y, th0, f, NAMES["nexi"], context=own_ctx)
+    np.testing.assert_array_equal(again["final_theta"], good["final_theta"])
