@@ -333,7 +333,7 @@ __global__ void __maxnreg__(96) fused_kernel_nexi(AdamParams a, int e_begin, int
 // Per voxel the operations of fused_kernel_nexi.  24 warps at 80 registers: 0-2 %
 // slower or faster by size, and from 25 tasks on only.
 // ---------------------------------------------------------------------------
-constexpr int kRotWarps = 20;              // 640 threads x 96 registers
+constexpr int kRotWarps = kTurnsBlock / 32;  // 20: 640 threads x 96 registers
 constexpr int kRotTasks = 96;              // tasks of a CTA, at most
 constexpr int kRotNodes = 1 << 18;         // epochs x shells x nodes of a unit, at most
 
@@ -1214,6 +1214,11 @@ static int nexi_span(const AdamParams& a, int e_begin, int e_end, int nvox, int 
         return 0;
     const int rounds = (int)((long long)((nvox / 32 + nsm - 1) / nsm) * epochs / (32 * kRotWarps));
     return std::max(1, std::min(rounds, kRotNodes / (a.P.nx * a.P.n_shell)));
+}
+
+bool fused_turns(const AdamParams& a, int model, int epochs) {
+    size_t smem;
+    return model == kNEXI && nexi_span(a, 1, epochs, a.nvtot, sm_count(), &smem) > 0;
 }
 
 template <int MODEL, int LOSS, bool STATS>

@@ -57,7 +57,7 @@ static gx_status fail(gx_status s, const char* fmt, ...) {
 // process (GACELLE_B200_AUTOTUNE=0 turns tuning off: the defaults are used).
 // ---------------------------------------------------------------------------
 struct TuneKey {
-    std::array<long long, 13> k;
+    std::array<long long, 17> k;
     bool operator<(const TuneKey& o) const { return k < o.k; }
 };
 static std::mutex g_tune_mu;
@@ -1063,8 +1063,11 @@ static gx_status upload_blk_table(AdamJob& J, int Bl, int** out) {
 }
 
 // Autotuner of the fused kernel's launch block.  Key: device, model, loss,
-// measurements, statistics / prior / weights / b1 / sigma-map variants,
-// optimiser, transform and the voxel-count class (log2 of the work-list).
+// measurements, flip angles, NEXI nodes, statistics / prior / weights / b1 /
+// sigma-map variants, optimiser, transform, the voxel-count class (log2 of the
+// work-list), and what the voxel count decides inside a class: which kernel
+// runs (the rules of fused_kind) and whether 32 threads are a
+// candidate.
 // On a miss every candidate (64, 128, 256, 512 threads, and 32 for short
 // work-lists, within the kernel's thread and shared-memory limits) runs a
 // few epochs of this job's own
@@ -1077,11 +1080,13 @@ static gx_status tune_fused(AdamJob& J) {
     int cls = 0;
     while ((1LL << (cls + 1)) <= (long long)J.nvtot) ++cls;
     const TuneKey key{{1, c->device, J.id, o->loss, J.nm, stats ? 1 : 0, J.prior ? 1 : 0, J.a.weights ? 1 : 0,
-                       J.a.b1 ? 1 : 0, J.a.sigma ? 1 : 0, o->optimiser, o->transform, cls}};
+                       J.a.b1 ? 1 : 0, J.a.sigma ? 1 : 0, o->optimiser, o->transform, cls,
+                       J.a.P.n_fa, J.a.P.nx, fused_kind(J.a, J.id, o->loss, J.B), J.nvtot <= 64 * 148 ? 1 : 0}};
     int Bl = o->iteration < 2 ? 128 : tune_lookup(key);  // trials need two epochs of history rows
     if (Bl <= 0) {
         const int N = o->iteration;
         AdamParams t = J.a;
+        t.wait_err = nullptr;  // the trials are of the kernel that has a block
         const size_t pn = (size_t)J.np * J.nvtot;
         float* sc;
         TRY(wsT(c, S_TUNE, 4 * pn, &sc));
@@ -1148,13 +1153,18 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
     const bool stop_possible = can_stop(o);
     const int chunk = stop_possible ? (o->chunk > 0 ? o->chunk : 200) : (N > 0 ? N : 1);
     TRY(alloc_outputs(J, out));
+    bool turns = false;  // the main pass's launches do not have a block to choose
     if (!J.tv && J.id == kNEXI && nexi_turns(J.nvtot, sm_count())) {
         TRY(wsT(c, S_WAIT_ERR, 1, &J.a.wait_err));
         CK(cudaMemsetAsync(J.a.wait_err, 0, sizeof(int), c->stream));
         J.a.wait_limit = c->hooks.wait_limit_cycles > 0 ? c->hooks.wait_limit_cycles : kFusedWaitClocks;
         J.a.wait_extra = c->hooks.barrier_extra_arrivals;
+        turns = fused_turns(J.a, J.id, std::min(chunk, N));
     }
-    if (J.autotune) TRY(tune_fused(J));
+    if (J.autotune && turns) {  // a last launch of one epoch and replays: the default block
+        J.Bl = 128;
+        TRY(upload_blk_table(J, J.Bl, &J.blk_l));
+    } else if (J.autotune) TRY(tune_fused(J));
     if (J.tv) {
         const char* env = getenv("GACELLE_B200_TV_KERNEL");
         bool want = !(env && strcmp(env, "step") == 0);
@@ -1246,7 +1256,7 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
     cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]);
     c->timing.main_kernel_ms = ms;
     c->timing.main_launches = n_main;
-    c->timing.block_size = J.Bl > 0 ? J.Bl : (J.use_persist ? J.plan.threads : J.B);
+    c->timing.block_size = turns ? kTurnsBlock : J.Bl > 0 ? J.Bl : (J.use_persist ? J.plan.threads : J.B);
     c->timing.autotuned = J.tuned_now ? 1 : 0;
     c->timing.tv_path = !J.use_persist ? 0
                         : GX_TV_PERSISTENT | (J.plan.quad_pairs ? GX_TV_PAIRS : 0) |
@@ -1702,8 +1712,8 @@ static int mcmc_nsamples(int iteration, int nb, int thinning) {
 
 // Autotuner of the MCMC kernels' block shape (Goodman-Weare: voxels per CTA;
 // MH: threads per CTA).  Key: device, model, algorithm, walkers, update
-// scheme, variables, measurements, weights / b1 variants and the voxel-count
-// class.  On a miss each candidate runs a few steps from the start on the
+// scheme, variables, measurements, flip angles, NEXI nodes, weights / b1
+// variants, whether the acceptance is screened, and the voxel-count class.  On a miss each candidate runs a few steps from the start on the
 // first voxels of this job (scratch walker state and sums; the job's buffers
 // untouched) and the fastest is cached for the process.
 static gx_status tune_mcmc(gx_context* c, const McmcParams& p, int model, int* block, bool* tuned) {
@@ -1711,7 +1721,7 @@ static gx_status tune_mcmc(gx_context* c, const McmcParams& p, int model, int* b
     while ((1LL << (cls + 1)) <= (long long)p.nvox) ++cls;
     const int W = p.algorithm == 1 ? p.nwalker : 1;
     const TuneKey key{{2, c->device, model, p.algorithm, W, p.update, p.nvar, p.nm, p.weights ? 1 : 0,
-                       p.b1 ? 1 : 0, cls, 0, 0}};
+                       p.b1 ? 1 : 0, cls, p.P.n_fa, p.P.nx, mcmc_screened(p, model) ? 1 : 0, 0, 0, 0}};
     int b = tune_lookup(key);
     if (b <= 0) {
         McmcParams t = p;

@@ -87,6 +87,9 @@ constexpr long long kFusedWaitClocks = 1LL << 32;
 // voxels may take the kernel whose waits need AdamParams::wait_err.
 int sm_count();
 bool nexi_turns(int nvtot, int nsm);
+// Whether launches of `epochs` epochs over the whole work-list take that kernel, and its block.
+bool fused_turns(const AdamParams& a, int model, int epochs);
+constexpr int kTurnsBlock = 640;
 // Largest launch block (multiple of 32) the fused kernel variant of this job
 // accepts: its thread limit and its per-block shared memory; 0 on error.
 int fused_block_limit(const AdamParams& a, int model, int loss, bool stats);
@@ -237,6 +240,7 @@ cudaError_t launch_mcmc_partners(const McmcParams& p, int* partner, cudaStream_t
 void gwg_launch_shape(const McmcParams& p, int block_hint, int* vpb, int* block, int* nblocks, size_t* smem);
 int mcmc_steps_per_launch(const McmcParams& p);
 int mcmc_mh_block(const McmcParams& p, int model, int block_hint);  // threads per block of a Metropolis-Hastings launch
+bool mcmc_screened(const McmcParams& p, int model);  // acceptance by the FP32 screen
 bool mcmc_batched(const McmcParams& p, int model);  // the kernel with a block of its own (no shape to tune)
 // Node table of a NEXI protocol (capi.cu); its place in dynamic shared memory.
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;

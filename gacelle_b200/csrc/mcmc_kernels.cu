@@ -1051,8 +1051,10 @@ static bool screened(const McmcParams& p) {
            p.ub[p.nvar - 1] <= kScreenMaxNoise;
 }
 
+bool mcmc_screened(const McmcParams& p, int model) { return model == kR2S && screened(p); }
+
 bool mcmc_batched(const McmcParams& p, int model) {
-    return p.algorithm == 0 && model == kR2S && screened(p) && p.nvox <= kMhBatchVoxels;
+    return p.algorithm == 0 && mcmc_screened(p, model) && p.nvox <= kMhBatchVoxels;
 }
 
 template <int MODEL>

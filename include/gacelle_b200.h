@@ -177,7 +177,7 @@ typedef struct {
     int32_t chunk;              /* fused path: iterations per launch if stopping may trigger; 0 = auto */
     /* threads per block; 0 = the default (128), or on the fused path without
      * TV the block chosen by the project's autotuner: the first call of a key
-     * (model, loss, measurement count, variant, optimiser, transform, voxel-
+     * (model, loss, protocol size, variant, optimiser, transform, kernel, voxel-
      * count class) times 64 / 128 / 256 / 512 threads (and 32 for work-lists
      * of at most 64 x 148 voxels) on a few epochs of its own data and the
      * fastest is kept for the process; GACELLE_B200_AUTOTUNE=0
@@ -275,7 +275,10 @@ typedef struct {
     int64_t kernel_launches;    /* launches of this library's kernels in the call */
     int64_t h2d_bytes, d2h_bytes;
     int32_t tv_path;            /* askAdam with TV: GX_TV_* flags of the main pass, else 0 */
-    int32_t block_size;         /* threads per block of the main kernel's launches */
+    int32_t block_size;         /* block of the main kernel's launches: its threads, or the voxels of a
+                                 * block where a thread takes two (the R2* and R1-R2* fits by MSE); 640
+                                 * where the NEXI kernel that takes voxels in turns runs, which has no
+                                 * block to choose */
     int32_t autotuned;          /* 1: the autotuner ran its trials in this call (block_size 0,
                                  * first call of its key in the process) */
     double aux_kernel_ms;       /* summed duration of the post-processing kernels (MCMC: the

@@ -310,3 +310,63 @@ def test_nexi_turns_wait_runs_out(own_ctx, chunk):
     _hooks(own_ctx)
     again = run_engine("nexi", y, th0, f, NAMES["nexi"], context=own_ctx)
     np.testing.assert_array_equal(again["final_theta"], good["final_theta"])
+
+
+@pytest.mark.parametrize("loss,sizes,over", [
+    ("rician", [100_003], {}), ("mse", [60_000, 45_003], {"convergenceStepTol": 1e-30, "convergenceGradTol": 1e-30})])
+def test_nexi_turns_forms(ctx, loss, sizes, over):
+    """NEXI fits in turns under the Rician loss, over several volumes and with a
+    chosen block equal those of the block kernel (one epoch a launch) bit for bit;
+    gx_timing.block_size tells which of the two ran."""
+    rng = np.random.default_rng(len(sizes))
+    gxm, om = models("nexi")
+    lb, ub = bounds("nexi")
+    data = []
+    for n in sizes:
+        s = oracle.forward(om, random_theta("nexi", n, rng))
+        data.append(np.abs(s + 0.02 * rng.standard_normal(s.shape)).astype(np.float32))
+    runs = []
+    for chunk in (0, 1):
+        f = fitting(iteration=9, chunk=chunk, lossFunction=loss, noiseSigma=0.02, **dict({"tol": -1e30 if loss == "rician" else 1e-30}, **over))
+        opts = gx_askadam.build_opts(f, NAMES["nexi"], lb, ub)
+        vols, res, keep = (_lib.GxVolume * len(sizes))(), (_lib.GxAskadamResult * len(sizes))(), []
+        for v, r, y in zip(vols, res, data):
+            n = y.shape[1]
+            th0 = np.tile(np.array([[0.4], [2.0], [1.0], [0.05]], np.float32), (1, n))
+            out = [np.zeros((4, n), np.float32), np.zeros((4, n), np.float32), np.zeros_like(y)]
+            v.nvox, v.dims[0], v.dims[1], v.dims[2] = n, n, 1, 1
+            v.data, v.theta0 = y.ctypes.data_as(_lib._fp), th0.ctypes.data_as(_lib._fp)
+            r.final_theta, r.min_theta, r.final_residual = (x.ctypes.data_as(_lib._fp) for x in out)
+            keep.append((th0, out))
+        _lib.check(_lib.lib().gx_askadam(ctx.ptr, C.byref(gxm.s), _lib.MEM_HOST, vols, len(sizes), C.byref(opts), res))
+        runs.append(([k[1] for k in keep], ctx.timing()["block_size"]))
+    (a, block_a), (b, block_b) = runs
+    assert block_a == 640 and block_b != 640
+    for x, y in zip(a, b):
+        for p, q in zip(x, y):
+            assert np.array_equal(p, q)
+
+
+def test_autotuner_keeps_kernels_apart(ctx):
+    """A block tuned for one kernel is not taken for another: fits of one
+    voxel-count class on either side of a rule, and protocols with as many
+    measurements but other flip angles, are tuned each; where the kernel has
+    no block to choose nothing is tuned."""
+    from helpers import run_engine
+
+    def tuned(kind, n, th0, **kw):
+        _, om = models(kind, **kw)
+        y = np.tile(oracle.forward(om, np.array(th0)[:, None]), (1, n)) + 0.01
+        r = run_engine(kind, y, np.tile(np.array(th0, np.float32)[:, None], (1, n)), fitting(iteration=3, tol=-np.inf),
+                       NAMES[kind], context=ctx, **kw)
+        return r["timing"]["autotuned"]
+
+    nexi = [0.4, 2.0, 1.0, 0.05]
+    assert [tuned("nexi", n, nexi, nx=11) for n in (100_003, 80_000, 80_100, 100_003)] == [0, 1, 0, 0]
+    te = np.linspace(2e-3, 40e-3, 11)
+    assert [tuned("r2s", n, [1.0, 30.0], te=te) for n in (70_000, 80_000, 70_100)] == [1, 1, 0]
+    for fa, nte in (([5.0, 20.0], 10), ([5.0, 10.0, 15.0, 20.0], 5)):
+        te = np.linspace(2e-3, 40e-3, nte)
+        assert tuned("r1r2s", 5000, [1.0, 1.0, 30.0], te=te, fa=fa) == 1
+    te = np.linspace(2e-3, 40e-3, 10)
+    assert [tuned("r1r2s", n, [1.0, 1.0, 30.0], te=te, fa=[5.0, 20.0]) for n in (8800, 9000, 9600)] == [1, 0, 1]
