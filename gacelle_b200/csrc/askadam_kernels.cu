@@ -325,7 +325,7 @@ __global__ void __maxnreg__(96) fused_kernel_nexi(AdamParams a, int e_begin, int
 // voxels, and its 20 warps take (task, epochs) units in turn: unit i is task
 // i % n, epochs i / n, by warp i % 20, so the warps stay busy until the last
 // round.  Between units a task's state lives in global memory; a unit waits for
-// the task's previous one (n units earlier, n > 20, of a warp of the same CTA:
+// the task's previous one (n units earlier, n >= 20, of a warp of the same CTA:
 // the least unfinished unit never waits, so all end), with a limit on the wait.
 // A wait lasts a unit at most, and a unit's epochs are bounded by its nodes
 // (kRotNodes, some 35 ms at 0.13 us a node and shell with 20 warps an SM), so that
@@ -1192,16 +1192,17 @@ int sm_count() {
     return n;
 }
 
-// Whether fused_kernel_nexi_turns may take a work-list: more than 20 tasks an SM
-// (fewer are resident at once anyway) and at most 96, beyond which a partial
-// wave of the block kernel weighs less than the turns' reloads.  Block kernel
+// Whether fused_kernel_nexi_turns may take a work-list: more tasks than the 20
+// an SM that are resident at once (the block kernel would start a second wave),
+// and at most 96 an SM, beyond which a partial wave of the block kernel weighs
+// less than the turns' reloads.  Every CTA then has 20 tasks or more.  Block kernel
 // -> turns, whole calls: 100,003 voxels x 100 nodes, Rician, 40 epochs (22
-// tasks) 16.3 -> 14.2 ms; 14 nodes, MSE, 100 epochs: 100,000 voxels 6.64 ->
-// 5.74, 150,000 8.29 -> 8.19, 328,050 (70 tasks) 18.2 -> 17.6; 640,000 voxels x
+// tasks) 16.3 -> 14.2 ms; 14 nodes, MSE, 60 epochs: 95,000 voxels (20.1 tasks) 5.02
+// -> 3.45, under the Rician loss 6.50 -> 4.35; 100 epochs: 100,000 voxels 6.64 -> 5.74, 150,000 8.29 -> 8.19, 328,050 (70 tasks) 18.2 -> 17.6; 640,000 voxels x
 // 60 epochs (136 tasks) 20.3 -> 20.6.
 bool nexi_turns(int nvtot, int nsm) {
     const int ntask = nvtot / 32;
-    return nsm > 0 && ntask / nsm > kRotWarps && (ntask + nsm - 1) / nsm <= kRotTasks;
+    return nsm > 0 && ntask > kRotWarps * nsm && (ntask + nsm - 1) / nsm <= kRotTasks;
 }
 
 // Epochs of a unit of fused_kernel_nexi_turns (about 32 rounds a launch, for a

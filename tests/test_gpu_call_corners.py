@@ -313,7 +313,8 @@ def test_nexi_turns_wait_runs_out(own_ctx, chunk):
 
 
 @pytest.mark.parametrize("loss,sizes,over", [
-    ("rician", [100_003], {}), ("mse", [60_000, 45_003], {"convergenceStepTol": 1e-30, "convergenceGradTol": 1e-30})])
+    ("rician", [100_003], {}), ("mse", [60_000, 45_003], {"convergenceStepTol": 1e-30, "convergenceGradTol": 1e-30}),
+    ("rician", [3, 99_000, 31], {"blockSize": 96}), ("mse", [94_752], {"blockSize": 32})])
 def test_nexi_turns_forms(ctx, loss, sizes, over):
     """NEXI fits in turns under the Rician loss, over several volumes and with a
     chosen block equal those of the block kernel (one epoch a launch) bit for bit;
