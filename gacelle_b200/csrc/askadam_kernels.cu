@@ -317,6 +317,18 @@ __global__ void __maxnreg__(96) fused_kernel_nexi(AdamParams a, int e_begin, int
     fused_body<MODEL, LOSS, STATS>(a, e_begin, e_end, update_last, record);
 }
 
+// The same for few voxels, whose time is one voxel's chain of nodes and not the
+// pipes': up to 128 registers (16 warps an SM), so that more of a node pair's
+// operations overlap.  Whole calls, 96 (112) -> 128 registers: 60 epochs x 14
+// nodes, 500-10,000 voxels MSE 1.38 (1.30) -> 1.22 ms, Rician 2.11 (2.00) -> 1.90;
+// 70,000 voxels 2.60 (2.55) -> 2.53 and 3.38 (3.34) -> 3.28; 20 epochs x 100
+// nodes, Rician, 500 voxels 2.47 (2.14) -> 1.97.
+template <int LOSS, bool STATS>
+__global__ void __maxnreg__(128) fused_kernel_nexi_wide(AdamParams a, int e_begin, int e_end, int update_last, int record) {
+    fused_body<kNEXI, LOSS, STATS>(a, e_begin, e_end, update_last, record);
+}
+constexpr int kWideWarps = 16, kWideBlock = 512;
+
 // ---------------------------------------------------------------------------
 // NEXI with lmax 0 when the voxels fill the resident warps a few times: the
 // blocks of fused_kernel_nexi run all epochs of their voxels, so a last wave
@@ -1197,13 +1209,17 @@ int sm_count() {
 // and at most 96 an SM, beyond which a partial wave of the block kernel weighs
 // less than the turns' reloads.  Every CTA then has 20 tasks or more.  Block kernel
 // -> turns, whole calls: 100,003 voxels x 100 nodes, Rician, 40 epochs (22
-// tasks) 16.3 -> 14.2 ms; 14 nodes, MSE, 60 epochs: 95,000 voxels (20.1 tasks) 5.02
-// -> 3.45, under the Rician loss 6.50 -> 4.35; 100 epochs: 100,000 voxels 6.64 -> 5.74, 150,000 8.29 -> 8.19, 328,050 (70 tasks) 18.2 -> 17.6; 640,000 voxels x
-// 60 epochs (136 tasks) 20.3 -> 20.6.
+// tasks) 16.3 -> 14.2 ms; 14 nodes, MSE, 60 epochs: 95,000 voxels (20.1
+// tasks) 5.02 -> 3.45, under the Rician loss 6.50 -> 4.35; 100 epochs: 100,000
+// voxels 6.64 -> 5.74, 150,000 8.29 -> 8.19, 328,050 (70 tasks) 18.2 -> 17.6;
+// 640,000 voxels x 60 epochs (136 tasks) 20.3 -> 20.6.
 bool nexi_turns(int nvtot, int nsm) {
     const int ntask = nvtot / 32;
     return nsm > 0 && ntask > kRotWarps * nsm && (ntask + nsm - 1) / nsm <= kRotTasks;
 }
+
+// Whether fused_kernel_nexi_wide takes a launch of nvox voxels: while all of them are resident at its registers.
+static bool nexi_wide(int nvox, int block, int nsm) { return block <= kWideBlock && nvox / 32 <= kWideWarps * nsm; }
 
 // Epochs of a unit of fused_kernel_nexi_turns (about 32 rounds a launch, for a
 // small last one, and no more than kRotNodes allows), or 0: not for this launch.
@@ -1242,6 +1258,8 @@ static cudaError_t fused_dispatch3(AdamParams a, int e_begin, int e_end, int upd
         }
     }
     auto k = fused_kernel_fn<MODEL, LOSS, STATS>();
+    if constexpr (MODEL == kNEXI)
+        if (nexi_wide(block * nblocks, block, sm_count())) k = fused_kernel_nexi_wide<LOSS, STATS>;
     if (kIsNexi<MODEL>) a.node_smem = nodes_fit(&smem);
     if (smem + sizeof(DevProtocol) > 48 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

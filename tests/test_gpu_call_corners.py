@@ -371,3 +371,21 @@ def test_autotuner_keeps_kernels_apart(ctx):
         assert tuned("r1r2s", 5000, [1.0, 1.0, 30.0], te=te, fa=fa) == 1
     te = np.linspace(2e-3, 40e-3, 10)
     assert [tuned("r1r2s", n, [1.0, 1.0, 30.0], te=te, fa=[5.0, 20.0]) for n in (8800, 9000, 9600)] == [1, 0, 1]
+
+
+@pytest.mark.parametrize("loss", ["mse", "rician", "l1"])
+@pytest.mark.parametrize("n,nx", [(1, 2), (33, 3), (700, 14), (75_700, 13), (75_800, 14), (300, 129)])
+def test_nexi_few_voxels(ctx, n, nx, loss):
+    """The NEXI kernel for few voxels (blocks up to 512 threads) gives the
+    parameters of the capped one (576 threads) bit for bit: odd and even node
+    counts, beyond the node table, around the voxel count of the rule."""
+    from helpers import run_engine
+    rng = np.random.default_rng(n)
+    _, om = models("nexi", nx=nx)
+    y = np.abs(oracle.forward(om, random_theta("nexi", n, rng)) + 0.01 * rng.standard_normal((24, n)))
+    th0 = np.tile(np.array([[0.4], [2.0], [1.0], [0.05]], np.float32), (1, n))
+    a, b, c = (run_engine("nexi", y, th0, fitting(iteration=6, blockSize=block, lossFunction=loss, tol=-1e30,
+                                                  noiseSigma=0.02), NAMES["nexi"], context=ctx, nx=nx)
+               for block in (128, 512, 576))
+    for k in ("final_theta", "min_theta", "final_residual"):
+        assert np.array_equal(a[k], c[k]) and np.array_equal(b[k], c[k]), k
