@@ -2044,7 +2044,8 @@ extern "C" gx_status gx_dictionary_match(gx_context* c, int32_t mem, const float
         TRY(wsT(c, S_DICT_STAT, 1, &stat));
     }
     CK(cudaEventRecord(c->ev[2], c->stream));
-    CK(launch_dictionary_match(ds, nvox, dd, ndict, nm, dw, ie, cj, db, dsse, op, list, stat, c->stream));
+    CK(launch_dictionary_match(ds, nvox, dd, ndict, nm, dw, ie, cj, db, dsse, op, list, stat,
+                               DictWait{c->hooks.wait_limit_cycles, c->hooks.barrier_extra_arrivals}, c->stream));
     CK(cudaEventRecord(c->ev[3], c->stream));
     if (mem == GX_MEM_HOST) {
         CK(cudaMemcpyAsync(best, db, sizeof(int32_t) * nvox, cudaMemcpyDeviceToHost, c->stream));

@@ -297,24 +297,25 @@ __host__ __device__ constexpr MmaPlan make_plan(int nc) {
     return plan;
 }
 
-constexpr long long kWaitCycles = 4000000000LL;  // bound of every wait: about 2 s
+constexpr long long kWaitCycles = 4000000000LL;  // bound of every wait: about 2 s (DictWait may shorten it)
 
 __device__ __forceinline__ unsigned int smem_addr(const void* p) { return (unsigned int)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool bar_wait(unsigned long long* bar, unsigned int parity) {
+__device__ __forceinline__ bool bar_wait(unsigned long long* bar, unsigned int parity, long long limit = kWaitCycles) {
     const long long t0 = clock64();
     do {
         unsigned int done;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
         if (done) return true;
-    } while (clock64() - t0 < kWaitCycles);
+    } while (clock64() - t0 < limit);
     return false;
 }
 
 // The same, ending early once another thread has raised err (looked at, with
 // the clock, every 16 tries).
-__device__ __forceinline__ bool bar_wait_or_err(unsigned long long* bar, unsigned int parity, volatile int* err) {
+__device__ __forceinline__ bool bar_wait_or_err(unsigned long long* bar, unsigned int parity, volatile int* err,
+                                                long long limit) {
     const long long t0 = clock64();
     do {
 #pragma unroll 1
@@ -324,7 +325,7 @@ __device__ __forceinline__ bool bar_wait_or_err(unsigned long long* bar, unsigne
                          : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
             if (done) return true;
         }
-    } while (!*err && clock64() - t0 < kWaitCycles);
+    } while (!*err && clock64() - t0 < limit);
     return false;
 }
 
@@ -374,6 +375,7 @@ __device__ __forceinline__ void tmem_load16(unsigned int addr, float (&r)[16]) {
 
 struct TensorSmem {
     unsigned long long full[2], done;   // operand tile arrived; products finished
+    unsigned long long drain;           // after a wait that ran out: all products finished
     unsigned int tmem;
     int err;
     int scan[kRows];                    // end of each voxel's items
@@ -389,7 +391,7 @@ struct TensorSmem {
 template <int NC>
 __global__ void __launch_bounds__(kTensorThreads, 2)
 dict_tensor_kernel(const float* signals, int nvox, const float* dict, int ndict, int nm, const double* invE,
-                   const unsigned char* op, int* best, float* best_sse, int* list, DictStat* stat) {
+                   const unsigned char* op, int* best, float* best_sse, int* list, DictStat* stat, DictWait wait) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TensorSmem S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -402,9 +404,9 @@ dict_tensor_kernel(const float* signals, int nvox, const float* dict, int ndict,
     if (tid == 0) {
         for (int b = 0; b < 2; ++b)
             asm volatile("mbarrier.init.shared.b64 [%0], 1;" :: "r"(smem_addr(&S.full[b])) : "memory");
-        asm volatile("mbarrier.init.shared.b64 [%0], 1;" :: "r"(smem_addr(&S.done)) : "memory");
+        asm volatile("mbarrier.init.shared.b64 [%0], %1;" :: "r"(smem_addr(&S.done)), "r"(1 + wait.extra) : "memory");
+        asm volatile("mbarrier.init.shared.b64 [%0], 1;" :: "r"(smem_addr(&S.drain)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        S.err = 0;
     }
     auto fetch = [&](int t) {  // operand tile t into buffer t & 1 (one thread)
         unsigned long long* bar = &S.full[t & 1];
@@ -414,8 +416,10 @@ dict_tensor_kernel(const float* signals, int nvox, const float* dict, int ndict,
                      : "memory");
     };
     int fetched = 0;  // tiles requested (thread 0)
-    if (tid == 0)
+    if (tid == 0) {
         for (; fetched < min(2, ntile); ++fetched) fetch(fetched);
+        S.err = *(volatile int*)&stat->err;  // an earlier CTA's wait ran out: the call has failed, no long waits here
+    }
     __syncwarp();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" :: "r"(smem_addr(&S.tmem)) : "memory");
@@ -448,7 +452,7 @@ dict_tensor_kernel(const float* signals, int nvox, const float* dict, int ndict,
     int kept = 0;
     for (int t = 0; t < ntile; ++t) {
         if (tid == 0) {
-            if (!bar_wait(&S.full[t & 1], (unsigned int)(t >> 1) & 1u)) S.err = 1;
+            if (!bar_wait(&S.full[t & 1], (unsigned int)(t >> 1) & 1u, wait.limit)) S.err = 1;
             else {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 mma_tile<NC>(tmem, smem_addr(opA) >> 4, smem_addr(opB + (size_t)(t & 1) * tb) >> 4);
@@ -456,7 +460,7 @@ dict_tensor_kernel(const float* signals, int nvox, const float* dict, int ndict,
                              :: "r"(smem_addr(&S.done)) : "memory");
             }
         }
-        const bool ok = __all_sync(0xffffffffu, bar_wait_or_err(&S.done, (unsigned int)t & 1u, &S.err));
+        const bool ok = __all_sync(0xffffffffu, bar_wait_or_err(&S.done, (unsigned int)t & 1u, &S.err, wait.limit));
         if (!ok) S.err = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok) {
@@ -496,8 +500,12 @@ dict_tensor_kernel(const float* signals, int nvox, const float* dict, int ndict,
     }
     S.best[tid] = top;
     S.nkeep[tid] = (unsigned char)kept;
-    if (tid == 0 && S.err)  // copies in flight, before the buffers are let go
+    if (tid == 0 && S.err) {  // copies and products in flight, before the buffers and the tensor memory are let go
         for (int t = max(0, fetched - 2); t < fetched; ++t) bar_wait(&S.full[t & 1], (unsigned int)(t >> 1) & 1u);
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                     :: "r"(smem_addr(&S.drain)) : "memory");
+        bar_wait(&S.drain, 0u);
+    }
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" :: "r"(tmem));
     if (S.err) {
@@ -681,7 +689,8 @@ size_t dict_operand_bytes(int ndict, int nm) { return (size_t)((ndict + kRows - 
 
 cudaError_t launch_dictionary_match(const float* signals, int nvox, const float* dict, int ndict, int nm,
                                     const float* wt, double* invE, double* Cj, int* best, float* best_sse,
-                                    unsigned char* op, int* list, DictStat* stat, cudaStream_t s) {
+                                    unsigned char* op, int* list, DictStat* stat, DictWait wait, cudaStream_t s) {
+    if (wait.limit <= 0) wait.limit = kWaitCycles;
     const bool tensor = op != nullptr;
     const int nentry = tensor ? (ndict + kRows - 1) / kRows * kRows : ndict;
     cudaError_t e = cudaSuccess;
@@ -704,7 +713,7 @@ cudaError_t launch_dictionary_match(const float* signals, int nvox, const float*
         e = cudaFuncSetAttribute(kt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         kt<<<(nvox - 1) / kRows + 1, kTensorThreads, smem, s>>>(signals, nvox, dict, ndict, nm, invE, op, best,
-                                                                    best_sse, list, stat);
+                                                                    best_sse, list, stat, wait);
         dict_scan_kernel<<<kFewLeft, kThreads, 0, s>>>(signals, nvox, dict, ndict, nm, invE, best, best_sse, list, stat);
         g_kernel_launches += 2;
         e = cudaGetLastError();

@@ -185,12 +185,18 @@ struct DictStat {
     int err;     // a bounded wait expired
     int pad;
 };
+// Test hooks of that kernel's waits: their bound (0: the default), and
+// arrivals more than are made that the wait for a tile's products asks for.
+struct DictWait {
+    long long limit;
+    int extra;
+};
 size_t dict_match_smem(int nm, bool weighted);
 bool dict_tensor_ok(int nvox, int ndict, int nm, bool weighted);
 size_t dict_operand_bytes(int ndict, int nm);
 cudaError_t launch_dictionary_match(const float* signals, int nvox, const float* dict, int ndict, int nm,
                                     const float* wt, double* invE, double* Cj, int* best, float* best_sse,
-                                    unsigned char* op, int* list, DictStat* stat, cudaStream_t s);
+                                    unsigned char* op, int* list, DictStat* stat, DictWait wait, cudaStream_t s);
 
 // Forward only (gx_forward).
 cudaError_t launch_forward_only(const DevProtocol& P, int model, const float* theta,

@@ -319,12 +319,13 @@ typedef struct {
      * an allocation failure would (GX_ENOMEM), without touching the device. */
     int32_t fail_alloc_at;
     /* > 0: bound, in SM clock cycles, of every wait in the persistent TV
-     * kernel and in the NEXI fit kernel whose warps take voxels in turns
-     * (default about 2 s). */
+     * kernel, in the NEXI fit kernel whose warps take voxels in turns and in
+     * the dictionary's tensor-core kernel (default about 2 s). */
     int64_t wait_limit_cycles;
     /* > 0: the persistent kernel's grid barrier waits for this many arrivals
      * more than the grid makes (the turns of the NEXI kernel for as many units
-     * more than are run), so its bounded wait runs out: every CTA then
+     * more than are run, a dictionary tile for as many arrivals more than its
+     * products make), so its bounded wait runs out: every CTA then
      * returns and the call reports GX_ETIMEOUT, with the context usable. */
     int32_t barrier_extra_arrivals;
 } gx_test_hooks;

@@ -389,3 +389,23 @@ def test_nexi_few_voxels(ctx, n, nx, loss):
                for block in (128, 512, 576))
     for k in ("final_theta", "min_theta", "final_residual"):
         assert np.array_equal(a[k], c[k]) and np.array_equal(b[k], c[k]), k
+
+
+def test_dictionary_wait_runs_out(own_ctx):
+    """A wait of the tensor-core kernel for products that nobody makes ends at
+    its limit: the call reports GX_ETIMEOUT and the next one matches."""
+    import time
+    rng = np.random.default_rng(5)
+    D = np.abs(rng.standard_normal((24, 1500))) + 0.1
+    y = D[:, rng.integers(0, 1500, 40_100)] + 0.01 * rng.standard_normal((24, 40_100))
+    good, sse, launches = _match(own_ctx, y, D)
+    assert launches == 4
+    _hooks(own_ctx, wait_limit_cycles=2_000_000, barrier_extra_arrivals=1)
+    t0 = time.perf_counter()
+    with pytest.raises(_lib.GacelleError) as e:
+        _match(own_ctx, y, D)
+    assert e.value.status == _lib.GX_ETIMEOUT and "dictionary" in str(e.value)
+    assert time.perf_counter() - t0 < 5.0
+    _hooks(own_ctx)
+    best, sse2, _ = _match(own_ctx, y, D)
+    assert np.array_equal(best, good) and np.array_equal(sse, sse2)
