@@ -13,6 +13,7 @@ startPoint, step, index-aligned), ``updateProperty``, ``fit`` and ``FWD``.
 from __future__ import annotations
 
 import ctypes as C
+import inspect
 
 import numpy as np
 
@@ -262,16 +263,22 @@ class gpuR2starMapping(_ModelBase):
         if not len(fitting["lb"]):
             fitting["lb"] = self.lb[: len(self.modelParams)]
         masked = None
-        if str(fitting["start"]).lower() == "prior" and data.ndim == 4 and tuple(data.shape[:3]) == utils.dims3(mask):
+        if str(fitting["start"]).lower() == "prior" and data.ndim == 4 and tuple(data.shape[:3]) == utils.dims3(mask) \
+                and self._stock("determine_x0", "estimate_prior", "R2star_trapezoidal"):
             masked = utils.to_GD(data, mask)
             pars0 = self._masked_prior(masked, fitting)
         else:
             pars0 = self.determine_x0(data, mask, fitting)
         w = None
-        if fitting["isWeighted"]:
+        if fitting["isWeighted"] or not self._stock("compute_optimisation_weights"):
             w = self.compute_optimisation_weights(data, fitting)
             w = None if np.all(w == 1) else w
         return self._solve(data, mask, w, pars0, fitting, masked=masked)
+
+    def _stock(self, *names):
+        """Whether these methods are this class's own: not overridden by a
+        subclass, nor replaced on the class or the instance."""
+        return all(n not in vars(self) and inspect.getattr_static(type(self), n) is _R2S_STOCK[n] for n in names)
 
     def _masked_prior(self, y, fitting):
         """determine_x0's prior start for the voxels of the mask alone (y: [Nmeas,
@@ -297,6 +304,9 @@ class gpuR2starMapping(_ModelBase):
         _rescale_m0(out, fitting, scale)
         _save(fitting, out)
         return out
+
+
+_R2S_STOCK = dict(vars(gpuR2starMapping))
 
 
 class despot1:
