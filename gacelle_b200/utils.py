@@ -29,7 +29,9 @@ def reshape_ND2GD(data, mask_idx) -> np.ndarray:
     data = np.asarray(data)
     d3 = dims3(data)
     flat = data.reshape((d3[0] * d3[1] * d3[2], -1), order="F")
-    return np.take(flat.T, mask_idx, axis=1)  # row by row: contiguous reads and writes
+    if isinstance(mask_idx, np.ndarray) and mask_idx.ndim == 1 and mask_idx.dtype.kind == "i":
+        return np.take(flat.T, mask_idx, axis=1)  # row by row: contiguous reads and writes
+    return np.ascontiguousarray(flat[mask_idx].T)  # booleans, slices
 
 
 def to_GD(data, mask, mask_idx=None) -> np.ndarray:

@@ -74,3 +74,16 @@ def test_overridden_weights_are_taken():
     assert np.all(_captured(Mine(TE), data, mask)["w"] == 0.5)
     assert _captured(models.gpuR2starMapping(TE), data, mask)["w"] is None
     assert np.any(_captured(models.gpuR2starMapping(TE), data, mask, isWeighted=True)["w"] != 1)
+
+
+@pytest.mark.parametrize("index", ["indices", "boolean", "slice", "list", "int32", "uint64", "negative"])
+def test_reshape_nd2gd_takes_any_row_index(index):
+    """Rows of the column-major voxel list by any of numpy's row indices."""
+    data, mask = _image()
+    flat = mask.ravel(order="F")
+    idx = {"indices": np.flatnonzero(flat), "boolean": flat, "slice": slice(3, 20, 2), "list": [5, 1, 7],
+           "int32": np.array([5, 1, 7], np.int32), "uint64": np.array([5, 1, 7], np.uint64),
+           "negative": np.array([-1, 0])}[index]
+    want = data.reshape((mask.size, -1), order="F")[idx].T
+    got = utils.reshape_ND2GD(data, idx)
+    assert got.flags.c_contiguous and np.array_equal(got, want)
