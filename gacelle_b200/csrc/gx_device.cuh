@@ -883,8 +883,8 @@ __device__ __forceinline__ void stage_protocol(const DevProtocol& P, DevProtocol
 }
 
 __device__ __forceinline__ void stage_nodes(const NexiNodes& src, NexiNodes* dst) {
-    const float4* f = src.a;
-    float4* t = dst->a;
+    const float4* f = reinterpret_cast<const float4*>(&src);  // the whole table: a[] and b[]
+    float4* t = reinterpret_cast<float4*>(dst);
     for (int i = threadIdx.x; i < (int)(sizeof(NexiNodes) / sizeof(float4)); i += blockDim.x) t[i] = f[i];
 }
 
