@@ -894,7 +894,7 @@ struct DsigAcc {
     float g[NP];
     __device__ __forceinline__ void add(int m, float S, const float (&dS)[NP]) {
         if (MayBeNonFinite<NP>::value && !isfinite(S)) return;  // as LossAcc does
-        float d = ds[m * s];
+        float d = ds[row(m, s)];
 #pragma unroll
         for (int k = 0; k < NP; ++k) g[k] += d * dS[k];
     }

@@ -635,6 +635,9 @@ static gx_status upload_surface(AdamJob& J, int* gidx) {
     return GX_OK;
 }
 
+// Whether an array [rows][n] has 32-bit indices.
+static bool rows_fit(int rows, long long n) { return rows * n <= 0x7fffffffLL; }
+
 static gx_status adam_setup(AdamJob& J) {
     gx_context* c = J.c;
     const gx_askadam_opts* o = J.o;
@@ -1150,6 +1153,10 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
     gx_context* c = J.c;
     const gx_askadam_opts* o = J.o;
     const int N = o->iteration;
+    // the TV kernels and the general kernel's residuals index [row][voxel] arrays in 32 bits
+    if ((J.tv || ((J.want_res_f || J.want_res_m) && fused_kind(J.a, J.id, o->loss, J.B) == kFusedGeneral)) &&
+        !rows_fit(std::max(J.nm, J.a.surf_maxnb), J.nvtot))
+        return fail(GX_EUNSUPPORTED, "more than 2^31 - 1 measurements x voxels with TV or residuals");
     const bool stop_possible = can_stop(o);
     const int chunk = stop_possible ? (o->chunk > 0 ? o->chunk : 200) : (N > 0 ? N : 1);
     TRY(alloc_outputs(J, out));
@@ -1824,6 +1831,8 @@ extern "C" gx_status gx_mcmc(gx_context* c, const gx_model* model, int32_t mem, 
         gx_mcmc_result& r = results[i];
         if (v.nvox < 1 || !v.data || !v.theta0) return fail(GX_EINVAL, "volume %d: need nvox, data and theta0 (pars0)", i);
         int nv = v.nvox;
+        if (o->algorithm == GX_MCMC_MH && !rows_fit(nm, nv))  // its kernels index the data in 32 bits
+            return fail(GX_EUNSUPPORTED, "volume %d: more than 2^31 - 1 measurements x voxels", i);
         McmcParams p;
         memset(&p, 0, sizeof(p));
         p.P = make_protocol(model, id, np, nm, nullptr, nullptr, 0);

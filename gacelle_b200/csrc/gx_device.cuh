@@ -273,6 +273,10 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 __device__ __forceinline__ float2 bcast2(float a) { return make_float2(a, a); }
 
+// Index of row m of an array [measurement][voxel] with `stride` voxels, in 64 bits: such an
+// array may hold more than 2^31 values.  (One widening product; a 64-bit stride costs several.)
+__device__ __forceinline__ long long row(int m, int stride) { return (long long)m * stride; }
+
 // Accumulates loss and d(loss)/d(theta) over the measurements of one voxel.
 // set_nan_inf_zero (utils/askadam.m:80): a non-finite prediction becomes 0
 // and carries no gradient.
@@ -856,7 +860,7 @@ template <int NP>
 struct SignalSink {
     float* out;   // out[m*os]
     int os;
-    __device__ __forceinline__ void add(int m, float S, const float (&)[NP]) { out[m * os] = S; }
+    __device__ __forceinline__ void add(int m, float S, const float (&)[NP]) { out[row(m, os)] = S; }
 };
 
 // Sum of weighted squared residuals, accumulated in FP64 (MCMC logP).

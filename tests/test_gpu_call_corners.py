@@ -409,3 +409,53 @@ def test_dictionary_wait_runs_out(own_ctx):
     _hooks(own_ctx)
     best, sse2, _ = _match(own_ctx, y, D)
     assert np.array_equal(best, good) and np.array_equal(sse, sse2)
+
+
+def test_arrays_of_more_than_2_31_values(own_ctx):
+    """Signals and gradients of arrays [measurement][voxel] with more than 2^31
+    values: every row holds what the same voxels give in a small call.  The
+    calls whose kernels index such arrays in 32 bits refuse them."""
+    import torch
+    n, few = (1 << 31) // 24 + 2000, 1000
+    gxm, _ = models("r1r2s")
+    lb, ub = bounds("r1r2s")
+    th = torch.from_numpy(random_theta("r1r2s", few, np.random.default_rng(0)).astype(np.float32)).cuda()
+    spread = torch.arange(n, device="cuda") % few
+    fp = lambda t: C.cast(C.c_void_p(t.data_ptr()), _lib._fp)  # noqa: E731
+    L = _lib.lib()
+    opts = gx_askadam.build_opts(fitting(lossFunction="l2", iteration=2), NAMES["r1r2s"], lb, ub)
+    out = {}
+    for m in (few, n):
+        t = th if m == few else th[:, spread].contiguous()
+        s = torch.zeros(24, m, device="cuda")
+        torch.cuda.synchronize()
+        _lib.check(L.gx_forward(own_ctx.ptr, C.byref(gxm.s), _lib.MEM_DEVICE, t.data_ptr(), None, m, s.data_ptr()))
+        vol, loss = _lib.GxVolume(), C.c_double()
+        vol.dims[0], vol.dims[1], vol.dims[2], vol.nvox, vol.data = m, 1, 1, m, fp(s)
+        g, r, t2 = torch.zeros_like(t), torch.zeros_like(s), (t * 1.05).contiguous()
+        torch.cuda.synchronize()
+        _lib.check(L.gx_model_gradient(own_ctx.ptr, C.byref(gxm.s), _lib.MEM_DEVICE, C.byref(vol), C.byref(opts),
+                                       t2.data_ptr(), g.data_ptr(), r.data_ptr(), C.byref(loss), None, None))
+        out[m] = [s, g * m, r]  # the gradient is of a mean over m voxels
+    for a, b in zip(out[few], out[n]):
+        for k in range(a.shape[0]):
+            assert torch.allclose(a[k][spread], b[k], rtol=1e-5, atol=1e-12), k
+    # refused before anything is read: Metropolis-Hastings, and a fit's residuals
+    x0 = torch.cat([t, torch.full((1, n), 0.02, device="cuda")]).contiguous()
+    vol.theta0 = fp(x0)
+    lo, hi, step = (np.array(v) for v in (list(lb) + [0.001], list(ub) + [0.1], [0.01, 0.01, 1.0, 0.005]))
+    o = _lib.GxMcmcOpts()
+    o.algorithm, o.iteration, o.thinning, o.burnin, o.repetition, o.nwalker = 0, 2, 1, 0.0, 1, 1
+    o.step_size, o.start_range, o.seed = 2.0, 0.001, 3
+    o.lb, o.ub, o.x_step = (v.ctypes.data_as(_lib._dp) for v in (lo, hi, step))
+    res, fit = _lib.GxMcmcResult(), _lib.GxAskadamResult()
+    res.mean, fit.final_residual, fit.final_theta, fit.min_theta = fp(x0), fp(r), fp(g), fp(g)
+    with pytest.raises(_lib.GacelleError) as e:
+        _lib.check(L.gx_mcmc(own_ctx.ptr, C.byref(gxm.s), _lib.MEM_DEVICE, C.byref(vol), 1, C.byref(o), C.byref(res)))
+    assert e.value.status == _lib.GX_EUNSUPPORTED
+    with pytest.raises(_lib.GacelleError) as e:
+        _lib.check(L.gx_askadam(own_ctx.ptr, C.byref(gxm.s), _lib.MEM_DEVICE, C.byref(vol), 1, C.byref(opts), C.byref(fit)))
+    assert e.value.status == _lib.GX_EUNSUPPORTED
+    out.clear()
+    del s, t, t2, g, r, x0, spread, a, b
+    torch.cuda.empty_cache()
