@@ -85,9 +85,10 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
     static_assert(NV == NP + 1, "the variables are the model's parameters and the noise sigma");
     double sos = 0.0;
     if constexpr (MODEL == kR2S) {
-        for (int m = 0; m < nm; ++m) {
+        for (int m = 0; m < P.nm; ++m) {
             const float r = r2s_residual(P.te_l2e[m], x[0], x[1], y[m * ys]);
-            sos += (double)mul1(mul1(w ? w[m * ws] : 1.0f, r), r);
+            const float ww = w ? w[m * ws] : 1.0f;
+            sos += (double)(ww * r * r);
         }
     } else {
         SosSink<NP> sink{y, ys, w, ws, 0.0};
