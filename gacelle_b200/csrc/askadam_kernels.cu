@@ -367,7 +367,7 @@ __global__ void __maxnreg__(96) fused_kernel_nexi_turns(AdamParams a, int e_begi
     stage_protocol(a.P, &s_P);
     stage_nodes(a.nodes, s_nodes);
     for (int i = tid; i < n; i += B) s_done[i] = 0;
-    if (tid == 0) s_err = *a.wait_err;  // an earlier launch's wait ran out: the call has failed
+    if (tid == 0) s_err = a.wait->err;  // an earlier launch's wait ran out: the call has failed
     __syncthreads();
     if (s_err) return;
     const int nspan = (e_end - e_begin + span) / span;
@@ -376,14 +376,15 @@ __global__ void __maxnreg__(96) fused_kernel_nexi_turns(AdamParams a, int e_begi
         if (c > 0) {
             int bad = 0;
             if (lane == 0) {
-                const long long start = clock64();
-                while (s_done[t] < c + a.wait_extra && !bad) {
+                const long long start = clock64(), limit = a.wait->limit;
+                const int need = c + a.wait->extra;
+                while (s_done[t] < need && !bad) {
                     __nanosleep(64);
-                    bad = s_err || clock64() - start > a.wait_limit;
+                    bad = s_err || clock64() - start > limit;
                 }
                 if (bad) {
                     s_err = 1;
-                    *a.wait_err = 1;
+                    a.wait->err = 1;
                 }
             }
             if (__shfl_sync(0xffffffffu, bad, 0)) return;
@@ -1226,7 +1227,7 @@ static bool nexi_wide(int nvox, int block, int nsm) { return block <= kWideBlock
 static int nexi_span(const AdamParams& a, int e_begin, int e_end, int nvox, int nsm, size_t* smem) {
     *smem = sizeof(NexiNodes) + sizeof(float) * (size_t)(32 * kRotWarps) * a.nm * (a.weights ? 2 : 1);
     const int epochs = e_end - e_begin + 1;
-    if (!a.wait_err || nvox != a.nvtot || !nexi_turns(nvox, nsm) || epochs < 2 || a.P.nx > kNodeTab ||
+    if (!a.wait || nvox != a.nvtot || !nexi_turns(nvox, nsm) || epochs < 2 || a.P.nx > kNodeTab ||
         *smem + sizeof(DevProtocol) + 1024 > kMaxSmemPerBlock)
         return 0;
     const int rounds = (int)((long long)((nvox / 32 + nsm - 1) / nsm) * epochs / (32 * kRotWarps));
@@ -1246,7 +1247,7 @@ static cudaError_t fused_dispatch3(AdamParams a, int e_begin, int e_end, int upd
                   sizeof(float) * (size_t)block * (a.nm * (a.weights ? 2 : 1) + 2 * a.P.n_fa);
     if constexpr (MODEL == kNEXI) {
         size_t turns;
-        const int nsm = a.wait_err ? sm_count() : 0;
+        const int nsm = a.wait ? sm_count() : 0;
         const int span = nexi_span(a, e_begin, e_end, block * nblocks, nsm, &turns);
         if (span > 0) {
             auto kt = fused_kernel_nexi_turns<LOSS, STATS>;

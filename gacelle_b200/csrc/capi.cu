@@ -91,7 +91,7 @@ enum Slot {
     S_MC_PART, S_MC_SUM, S_MC_SUMSQ, S_MC_SHIFT, S_MC_X0, S_MC_POST, S_MC_ACC, S_MC_MEAN,
     S_MC_STD, S_FWD_TH, S_FWD_SIG, S_FWD_B1, S_BAR, S_MC_GLOB, S_ROBUST, S_DICT_SIG, S_DICT_D,
     S_DICT_W, S_DICT_OP, S_DICT_LIST, S_DICT_STAT, S_DICT_E, S_DICT_C, S_DICT_B, S_DICT_S, S_FLAGS, S_DATA_QUADS, S_PRIOR_MU, S_PRIOR_SD, S_SURF_NB, S_SURF_LEN,
-    S_MC_STATS, S_MC_X, S_MC_LP, S_TUNE, S_TUNE_HIST, S_BLK_L, S_WAIT_ERR, S_HGRID0, S_HGRID1, S_NSLOTS
+    S_MC_STATS, S_MC_X, S_MC_LP, S_TUNE, S_TUNE_HIST, S_BLK_L, S_WAIT, S_HGRID0, S_HGRID1, S_NSLOTS
 };
 
 struct gx_context {
@@ -1006,7 +1006,7 @@ static gx_status replay_volume(AdamJob& J, int i, int target, float* th_out, flo
     AdamParams base = J.a;
     base.z = J.zr; base.m1 = J.m1r; base.m2 = J.m2r;
     base.zprev = nullptr;
-    base.wait_err = nullptr;
+    base.wait = nullptr;
     base.ckpt_every = 0;
     View V;
     TRY(make_view(J, i, base, &V));
@@ -1089,7 +1089,7 @@ static gx_status tune_fused(AdamJob& J) {
     if (Bl <= 0) {
         const int N = o->iteration;
         AdamParams t = J.a;
-        t.wait_err = nullptr;  // the trials are of the kernel that has a block
+        t.wait = nullptr;  // the trials are of the kernel that has a block
         const size_t pn = (size_t)J.np * J.nvtot;
         float* sc;
         TRY(wsT(c, S_TUNE, 4 * pn, &sc));
@@ -1162,10 +1162,10 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
     TRY(alloc_outputs(J, out));
     bool turns = false;  // the main pass's launches do not have a block to choose
     if (!J.tv && J.id == kNEXI && nexi_turns(J.nvtot, sm_count())) {
-        TRY(wsT(c, S_WAIT_ERR, 1, &J.a.wait_err));
-        CK(cudaMemsetAsync(J.a.wait_err, 0, sizeof(int), c->stream));
-        J.a.wait_limit = c->hooks.wait_limit_cycles > 0 ? c->hooks.wait_limit_cycles : kFusedWaitClocks;
-        J.a.wait_extra = c->hooks.barrier_extra_arrivals;
+        TRY(wsT(c, S_WAIT, 1, &J.a.wait));
+        const FusedWait w{0, c->hooks.barrier_extra_arrivals,
+                          c->hooks.wait_limit_cycles > 0 ? c->hooks.wait_limit_cycles : kFusedWaitClocks};
+        CK(cudaMemcpyAsync(J.a.wait, &w, sizeof(w), cudaMemcpyHostToDevice, c->stream));
         turns = fused_turns(J.a, J.id, std::min(chunk, N));
     }
     if (J.autotune && turns) {  // a last launch of one epoch and replays: the default block
@@ -1273,9 +1273,9 @@ static gx_status adam_fused(AdamJob& J, AdamOut& out) {
         CK(cudaMemcpy(&hb, J.barrier, sizeof(hb), cudaMemcpyDeviceToHost));
         if (hb.error) return fail(GX_ETIMEOUT, "askAdam TV kernel: a grid barrier wait expired");
     }
-    if (J.a.wait_err) {
+    if (J.a.wait) {
         int expired = 0;
-        CK(cudaMemcpyAsync(&expired, J.a.wait_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(&expired, &J.a.wait->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         if (expired) return fail(GX_ETIMEOUT, "askAdam fused kernel: a wait expired");
     }

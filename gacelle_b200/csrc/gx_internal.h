@@ -28,6 +28,14 @@ struct DevVol {
     float prior_off;    // prior regulariser loss of the grid points outside the mask
 };
 
+// Device-side state of the waits in a fused kernel (beside AdamParams, whose size the
+// persistent TV kernel's time depends on: 16 bytes more, 0.8 %).
+struct FusedWait {
+    int err;          // set when a wait ran out
+    int extra;        // spans more than are made that a wait asks for (test hook)
+    long long limit;  // clocks of a wait, at most
+};
+
 // Parameters shared by the askAdam kernels (passed by value).
 struct AdamParams {
     DevProtocol P;
@@ -52,9 +60,7 @@ struct AdamParams {
     float* ckpt;                  // checkpoint slots, each 3*np*nvtot floats
     int ckpt_every;
     float* res_out;               // [nm][nvtot] or nullptr
-    int* wait_err;                // set by a fused kernel whose wait ran out; nullptr: kernels without waits only
-    long long wait_limit;         // clocks of such a wait, at most
-    int wait_extra;               // spans more than are made that it asks for (test hook)
+    FusedWait* wait;              // of the fused kernel with waits; nullptr: kernels without only
     // TV
     int n_reg;
     int reg_param[kMaxReg];
@@ -84,7 +90,7 @@ cudaError_t launch_fused(const AdamParams& a, int model, int loss, bool stats, i
 // Bound of the waits in fused kernels, about 2 s: kRotNodes keeps what they wait for far below it.
 constexpr long long kFusedWaitClocks = 1LL << 32;
 // Multiprocessors of the current device; whether a NEXI fit of nvtot padded
-// voxels may take the kernel whose waits need AdamParams::wait_err.
+// voxels may take the kernel whose waits need AdamParams::wait.
 int sm_count();
 bool nexi_turns(int nvtot, int nsm);
 // Whether launches of `epochs` epochs over the whole work-list take that kernel, and its block.
