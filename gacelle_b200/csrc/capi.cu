@@ -1558,7 +1558,8 @@ extern "C" gx_status gx_askadam(gx_context* c, const gx_model* model, int32_t me
 }
 
 // The evaluation without a regulariser: one kernel on the caller's device
-// arrays, or on contiguous device copies of host arrays; no fit state is set up.
+// arrays, or on contiguous device copies of host arrays and of device arrays
+// that an output overlaps; no fit state is set up.
 static gx_status gradient_direct(AdamJob& J, const float* theta, float* gtheta, float* residual, double* loss,
                                  double* loss_fid, double* loss_reg, long long launches0) {
     gx_context* c = J.c;
@@ -1578,10 +1579,16 @@ static gx_status gradient_direct(AdamJob& J, const float* theta, float* gtheta, 
     a.huber_delta = (float)o->huber_delta;
     a.sigma_default = (float)o->sigma;
     const bool host = copy_kind_host(J.mem);
-    // a host array's copy on the device, or the caller's device array
+    // whether an output's range meets the input's (in-place calls): the kernel
+    // reads the inputs while others of its threads write
+    auto meets = [&](const float* p, int rows, const float* out, int out_rows) {
+        const uintptr_t a0 = (uintptr_t)p, b0 = (uintptr_t)out;
+        return out && a0 < b0 + sizeof(float) * out_rows * n && b0 < a0 + sizeof(float) * rows * n;
+    };
+    // the device's copy of a host array or of one that an output meets, or the caller's device array
     auto in = [&](Slot s, const float* p, int rows, const float** out) -> gx_status {
         *out = p;
-        if (!host || !p) return GX_OK;
+        if (!p || (!host && !meets(p, rows, gtheta, J.np) && !meets(p, rows, residual, J.nm))) return GX_OK;
         float* d;
         TRY(wsT(c, s, rows * n, &d));
         TRY(upload_rows(c, d, n, 0, p, rows, (int)n, J.mem, &J.h2d));

@@ -459,3 +459,39 @@ def test_arrays_of_more_than_2_31_values(own_ctx):
     out.clear()
     del s, t, t2, g, r, x0, spread, a, b
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("loss", ["mse", "l1"])
+@pytest.mark.parametrize("kind", ["r2s", "r1r2s", "nexi"])
+@pytest.mark.parametrize("shift", [0, 1, 5, "row"])
+def test_gradient_in_place(ctx, kind, loss, shift):
+    """Residual written over the data, and gradient over the parameters, whole
+    or shifted by some values or a row: the results of separate arrays."""
+    import torch
+    rng = np.random.default_rng(4)
+    n = 3000
+    gxm, om = models(kind)
+    lb, ub = bounds(kind)
+    opts = gx_askadam.build_opts(fitting(lossFunction=loss), NAMES[kind], lb, ub)
+    th = random_theta(kind, n, rng).astype(np.float32)
+    th[0, 7] = np.nan
+    s = oracle.forward(om, random_theta(kind, n, rng))
+    y = (s + 0.02 * rng.standard_normal(s.shape)).astype(np.float32)
+    fp = lambda a: C.cast(C.c_void_p(a), _lib._fp)  # noqa: E731
+
+    def call(off):
+        pad = 0 if off is None else off
+        ty, tt = (torch.zeros(x.size + pad, device="cuda") for x in (y, th))
+        ty[:y.size], tt[:th.size] = torch.from_numpy(y.ravel()).cuda(), torch.from_numpy(th.ravel()).cuda()
+        r, g = (torch.zeros_like(ty), torch.zeros_like(tt)) if off is None else (ty, tt)
+        vol, loss_out = _lib.GxVolume(), C.c_double()
+        vol.dims[0], vol.dims[1], vol.dims[2], vol.nvox, vol.data = n, 1, 1, n, fp(ty.data_ptr())
+        torch.cuda.synchronize()
+        _lib.check(_lib.lib().gx_model_gradient(ctx.ptr, C.byref(gxm.s), _lib.MEM_DEVICE, C.byref(vol), C.byref(opts),
+                                                tt.data_ptr(), g.data_ptr() + 4 * pad, r.data_ptr() + 4 * pad,
+                                                C.byref(loss_out), None, None))
+        return r[pad:pad + y.size].cpu().numpy(), g[pad:pad + th.size].cpu().numpy(), loss_out.value
+
+    a, b = call(None), call(n if shift == "row" else shift)
+    assert np.array_equal(a[0], b[0], equal_nan=True) and np.array_equal(a[1], b[1], equal_nan=True)
+    assert np.isclose(a[2], b[2], rtol=1e-12)
