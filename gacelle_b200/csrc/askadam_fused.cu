@@ -151,7 +151,8 @@ __global__ void fused_r2s_kernel(AdamParams a, int e_begin, int e_end, int updat
 // operations a parameter, 61 % of the epoch at R1-R2*, whose epoch took three
 // times the instructions with one voxel a thread).  1.26 M voxels in six volumes, joint
 // R1-R2*, 12 echoes x 2 angles, 400 epochs: 8.38 -> 4.93 ms (110 registers
-// uncapped: 5.06, 64: 5.36).  R2*, 12 echoes, 500 epochs of 640,000 voxels:
+// uncapped: 5.06, 64: 5.36); with stopping statistics (68 bytes spilled) one volume
+// of as many voxels, whole call, 9.6 -> 6.6 ms.  R2*, 12 echoes, 500 epochs of 640,000 voxels:
 // 2.21 ms one voxel a thread -> 1.73 ms.
 // Two voxels a thread: thread t of a block takes voxels base + 64 (t / 32) +
 // t % 32 and that + 32, lane .x and .y of the pair instructions.

@@ -1094,8 +1094,8 @@ struct GradAcc {
 // pass, so that the measurements and parameters are read once and gradient and
 // residual written once (the op-by-op kernels passed signal and its derivative
 // through memory).  Bound by those bytes for R2* and R1-R2*, by the node loop
-// for NEXI.  230,000 voxels x 24 measurements, joint R1-R2*, a call: 180 us
-// (padded copies, an unused start state, three passes) -> 50 us.
+// for NEXI.  230,000 voxels x 24 measurements, joint R1-R2*, a call: 185 us
+// (padded copies, an unused start state, three passes) -> 57 us.
 template <int MODEL, int LOSS>
 __global__ void gradient_kernel(AdamParams a, const float* theta, float* gtheta, float norm, double normd, double* total) {
     constexpr int NP = ModelNP<MODEL>::value;

@@ -241,7 +241,8 @@ dict_match_kernel(const float* signals, int nvox, const float* dict, int ndict, 
 // 60 k clocks of a block's 240 k; two CTAs share an SM so that one works under
 // the other's waits.  500,000 voxels x 10^4 entries x 24 measurements: 14.6 ms
 // (FP64 pipe 47 %, operands from shared memory) -> 2.4 ms; 20,000 x 2000:
-// 0.11 ms; 1000 x 10^4: 0.17 ms.  The products are unrolled with descriptors
+// 0.11 ms; 1000 x 10^4: 0.17 ms; 200,000 x 10^4 x 64 (280 bytes spilled): 13.7
+// -> 2.7 ms.  The products are unrolled with descriptors
 // known at compile time: with descriptors loaded in a loop the issuing thread
 // took 126 clocks a product, unrolled it takes the pipe's 62.
 // ---------------------------------------------------------------------------

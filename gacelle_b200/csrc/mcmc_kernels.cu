@@ -124,7 +124,8 @@ __device__ __forceinline__ double log_prob_t(int nm, const DevProtocol& P, const
 // Measurements in registers, echo constants in the constant bank; kernels for
 // up to 8, 12 and 16 echoes, since a test per echo and one chain of sums cost a
 // tenth of the kernel.  12,013 voxels x 50 walkers x 500
-// steps, 12 echoes: 6.93 (all FP64) -> 3.65 ms; Metropolis-Hastings, 4096
+// steps, 12 echoes: 6.93 (all FP64) -> 3.65 ms; red-black, 12,000 x 50 x 300,
+// whole call: 6.50 -> 3.72 ms (124-152 bytes spilled); Metropolis-Hastings, 4096
 // voxels x 10,000 steps: 15.4 -> 6.1 ms (one dependent chain a voxel, 1.4-2.1
 // -> 0.6 us a step).
 constexpr int kScreenM = 16;
