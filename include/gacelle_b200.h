@@ -339,14 +339,22 @@ gx_status gx_model_sizes(const gx_model* model, int32_t* nparam, int32_t* nmeas)
 gx_status gx_forward(gx_context* ctx, const gx_model* model, int32_t mem, const float* theta,
                      const float* aux, int32_t nvox, float* signal);
 
+/* One evaluation of loss and d loss / d theta (utils/askadam.m:23-117) at any
+ * theta.  A prediction that is not finite counts as 0 with the derivative 0
+ * (set_nan_inf_zero, utils/askadam.m:80).  gtheta and residual may be NULL, and
+ * may overlap the inputs. */
 gx_status gx_model_gradient(gx_context* ctx, const gx_model* model, int32_t mem,
                             const gx_volume* vol, const gx_askadam_opts* opts,
                             const float* theta, float* gtheta, float* residual,
                             double* loss, double* loss_fidelity, double* loss_reg);
 
+/* GX_EUNSUPPORTED for a work-list of more than 2^31 - 1 measurements x voxels
+ * with TV, or with residuals where the general fused kernel runs. */
 gx_status gx_askadam(gx_context* ctx, const gx_model* model, int32_t mem, const gx_volume* vols,
                      int32_t nvol, const gx_askadam_opts* opts, gx_askadam_result* results);
 
+/* GX_EUNSUPPORTED for Metropolis-Hastings on a volume of more than 2^31 - 1
+ * measurements x voxels. */
 gx_status gx_mcmc(gx_context* ctx, const gx_model* model, int32_t mem, const gx_volume* vols,
                   int32_t nvol, const gx_mcmc_opts* opts, gx_mcmc_result* results);
 
