@@ -1727,7 +1727,8 @@ static int mcmc_nsamples(int iteration, int nb, int thinning) {
 // Autotuner of the MCMC kernels' block shape (Goodman-Weare: voxels per CTA;
 // MH: threads per CTA).  Key: device, model, algorithm, walkers, update
 // scheme, variables, measurements, flip angles, NEXI nodes, weights / b1
-// variants, whether the acceptance is screened, and the voxel-count class.  On a miss each candidate runs a few steps from the start on the
+// variants, whether the acceptance is screened, and the voxel-count class.  On
+// a miss each candidate runs a few steps from the start on the
 // first voxels of this job (scratch walker state and sums; the job's buffers
 // untouched) and the fastest is cached for the process.
 static gx_status tune_mcmc(gx_context* c, const McmcParams& p, int model, int* block, bool* tuned) {
